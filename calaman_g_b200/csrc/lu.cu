@@ -25,11 +25,11 @@
 // permutation and runs blocked forward / backward substitution (diagonal
 // blocks per warp, off-diagonal blocks on the GEMM).
 #include <cooperative_groups.h>
-#include <cfloat>
 #include <climits>
 #include <type_traits>
 
 #include "kernels.cuh"
+#include "lu_panel.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -122,12 +122,6 @@ __device__ __forceinline__ void cp_async_elem(T *dst, const T *src) {
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::);
 }
-
-template <typename T> __device__ __forceinline__ double safe_min();
-template <> __device__ __forceinline__ double safe_min<float>() { return FLT_MIN; }
-template <> __device__ __forceinline__ double safe_min<double>() { return DBL_MIN; }
-template <> __device__ __forceinline__ double safe_min<float2>() { return FLT_MIN; }
-template <> __device__ __forceinline__ double safe_min<double2>() { return DBL_MIN; }
 
 __device__ __noinline__ void panel_finish(cg::cluster_group &cluster, int rank, int k, int kb,
                                           const int *plist, const int *flags, int *mpos, int *morg,
@@ -421,216 +415,6 @@ __device__ __noinline__ void panel_finish(cg::cluster_group &cluster, int rank, 
   cluster.sync();
 }
 
-// ---------------------------------------------------------------------------
-// Register-resident panel: the algorithm of lu_panel_kernel with each row of
-// the panel held in the registers of NCPH adjacent lanes (lane phase q keeps
-// columns q, q + NCPH, ...), so the rank-1 update costs no shared-memory
-// traffic; only the pivot row is broadcast from shared memory. The CTA whose
-// candidate wins already publishes the pivot's reciprocal with the row, so
-// the division is done once, by one thread, while the row is being copied.
-// Used when the rows of a CTA fit its NT / NCPH lanes.
-// ---------------------------------------------------------------------------
-template <typename T, int KB, int NCPH, int NT>
-__global__ void __launch_bounds__(NT)
-    lu_panel_reg_kernel(int n, T *__restrict__ A, int lda, int k, int kb, int rpc,
-                        int *__restrict__ ipiv, int *__restrict__ perm, int *__restrict__ g_map_pos,
-                        int *__restrict__ g_map_src, int *__restrict__ g_map_count,
-                        int *__restrict__ info) {
-  constexpr int CPL = KB / NCPH;  // columns per lane
-  cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank();
-  const int ncta = (int)cluster.num_blocks();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nwarps = blockDim.x >> 5;
-  const int h = n - k;
-  const int r0 = rank * rpc;
-  int rows_here = h - r0;
-  rows_here = rows_here < 0 ? 0 : (rows_here > rpc ? rpc : rows_here);
-
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const PanelSmem o = panel_smem<T>(0, KB);
-  T *slot_row = reinterpret_cast<T *>(smem_raw + o.slot_row);    // [2][KB]
-  T *slot_diag = reinterpret_cast<T *>(smem_raw + o.slot_diag);  // [2][KB]
-  T *cand = reinterpret_cast<T *>(smem_raw + o.cand);            // [kMaxCluster][KB]
-  T *oldrow = reinterpret_cast<T *>(smem_raw + o.oldrow);
-  T *slot_rcp = reinterpret_cast<T *>(smem_raw + o.slot_rcp);
-  T *cand_rcp = reinterpret_cast<T *>(smem_raw + o.cand_rcp);
-  double *slot_val = reinterpret_cast<double *>(smem_raw + o.slot_val);
-  int *slot_idx = reinterpret_cast<int *>(smem_raw + o.slot_idx);
-  double *cand_val = reinterpret_cast<double *>(smem_raw + o.cand_val);
-  int *cand_idx = reinterpret_cast<int *>(smem_raw + o.cand_idx);
-  double *red_val = reinterpret_cast<double *>(smem_raw + o.red_val);
-  int *red_idx = reinterpret_cast<int *>(smem_raw + o.red_idx);
-  int *plist = reinterpret_cast<int *>(smem_raw + o.plist);
-  int *flags = reinterpret_cast<int *>(smem_raw + o.flags);
-
-  const int phase = tid % NCPH;
-  const int li = tid / NCPH;  // this lane's row within the CTA
-  const bool has_row = li < rows_here;
-  const int gi = r0 + li;     // panel-relative row
-  const int group0 = lane & ~(NCPH - 1);
-
-  // ---- stage: this lane's columns of its row ----
-  T r[CPL];
-#pragma unroll
-  for (int u = 0; u < CPL; ++u) {
-    const int c = phase + u * NCPH;
-    r[u] = (has_row && c < kb) ? A[(std::size_t)(k + c) * lda + (k + gi)] : elem<T>::zero();
-  }
-  if (tid == 0) flags[0] = -1;
-
-  // candidate for column 0: the phase-0 lane of every row
-  double bv = -1.0;
-  int bi = INT_MAX;
-  if (has_row && phase == 0) argmax_merge(bv, bi, abs1(r[0]), gi);
-
-  for (int j = 0; j < kb; ++j) {
-    const int par = j & 1;
-    const int owner_j = j / rpc;
-    const int jphase = j % NCPH, ju = j / NCPH;
-    // ---- (1) CTA-wide candidate; the lanes holding it publish its row ----
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const double ov = __shfl_xor_sync(0xffffffffu, bv, off);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-      argmax_merge(bv, bi, ov, oi);
-    }
-    if (lane == 0) {
-      red_val[warp] = bv;
-      red_idx[warp] = bi;
-    }
-    __syncthreads();
-    double cv = lane < nwarps ? red_val[lane] : -1.0;
-    int ci = lane < nwarps ? red_idx[lane] : INT_MAX;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const double ov = __shfl_xor_sync(0xffffffffu, cv, off);
-      const int oi = __shfl_xor_sync(0xffffffffu, ci, off);
-      argmax_merge(cv, ci, ov, oi);
-    }
-    if (tid == 0) {
-      slot_val[par] = cv;
-      slot_idx[par] = ci;
-    }
-    if (has_row && (gi == ci || gi == j)) {
-#pragma unroll
-      for (int u = 0; u < CPL; ++u) {
-        const int c = phase + u * NCPH;
-        if (c < kb) {
-          if (gi == ci) slot_row[par * KB + c] = r[u];
-          if (gi == j) slot_diag[par * KB + c] = r[u];
-        }
-      }
-      if (gi == ci && phase == jphase) {  // one division per column, off the other lanes' path
-        T x = elem<T>::zero();
-#pragma unroll
-        for (int u = 0; u < CPL; ++u)
-          if (u == ju) x = r[u];
-        slot_rcp[par] = is_zero(x) ? elem<T>::one() : divide(elem<T>::one(), x);
-      }
-    }
-    cluster.sync();
-
-    // ---- (2) one DSMEM round trip: every candidate, its row, and row j ----
-    for (int t = tid; t < (kMaxCluster + 1) * KB + kMaxCluster; t += blockDim.x) {
-      if (t < kMaxCluster * KB) {
-        const int q = t / KB, c = t % KB;  // KB is a power of two
-        if (q < ncta && c < kb) cand[q * KB + c] = cluster.map_shared_rank(slot_row, q)[par * KB + c];
-      } else if (t < (kMaxCluster + 1) * KB) {
-        const int c = t - kMaxCluster * KB;
-        if (c < kb) oldrow[c] = cluster.map_shared_rank(slot_diag, owner_j)[par * KB + c];
-      } else {
-        const int q = t - (kMaxCluster + 1) * KB;
-        if (q < ncta) {
-          cand_val[q] = cluster.map_shared_rank(slot_val, q)[par];
-          cand_idx[q] = cluster.map_shared_rank(slot_idx, q)[par];
-          cand_rcp[q] = cluster.map_shared_rank(slot_rcp, q)[par];
-        }
-      }
-    }
-    __syncthreads();
-
-    // ---- (3) the pivot ----
-    double pv = lane < ncta ? cand_val[lane] : -1.0;
-    int p = lane < ncta ? cand_idx[lane] : INT_MAX;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const double ov = __shfl_xor_sync(0xffffffffu, pv, off);
-      const int oi = __shfl_xor_sync(0xffffffffu, p, off);
-      argmax_merge(pv, p, ov, oi);
-    }
-    bool forced = false;
-    if (p == INT_MAX || p < j) {  // no comparable candidate (NaN column): keep row j
-      p = j;
-      pv = 0.0;
-      forced = true;
-    }
-    const int powner = p / rpc;
-    const T *pivrow = (p == j) ? oldrow : cand + powner * KB;
-    const T piv = pivrow[j];
-    const bool singular = forced || is_zero(piv);
-    const bool use_recip = abs1(piv) >= safe_min<T>();
-    const T rpiv = cand_rcp[powner];
-    if (tid == 0) {
-      plist[j] = p;
-      if (pv == 0.0 && flags[0] < 0) flags[0] = j;
-    }
-
-    // ---- (4) swap, scale, rank-1 update, next candidate: all in registers ----
-    T xj_mine = elem<T>::zero();
-#pragma unroll
-    for (int u = 0; u < CPL; ++u)
-      if (u == ju) xj_mine = r[u];
-    T xj = shfl(xj_mine, group0 + jphase);
-    bv = -1.0;
-    bi = INT_MAX;
-    if (has_row && gi >= j) {
-      if (gi == j) {  // position j receives the pivot row
-#pragma unroll
-        for (int u = 0; u < CPL; ++u) {
-          const int c = phase + u * NCPH;
-          if (c < kb) r[u] = pivrow[c];
-        }
-      } else {
-        if (gi == p) {  // position p receives the old row j
-          xj = oldrow[j];
-#pragma unroll
-          for (int u = 0; u < CPL; ++u) {
-            const int c = phase + u * NCPH;
-            if (c < kb) r[u] = oldrow[c];
-          }
-        }
-        const T l = singular ? xj : (use_recip ? mul(xj, rpiv) : divide(xj, piv));
-#pragma unroll
-        for (int u = 0; u < CPL; ++u) {
-          const int c = phase + u * NCPH;
-          if (c == j) r[u] = l;
-          else if (c > j && c < kb) r[u] = sub(r[u], mul(l, pivrow[c]));
-        }
-        if (j + 1 < kb && phase == (j + 1) % NCPH) {
-          const int nu = (j + 1) / NCPH;
-          T xn = elem<T>::zero();
-#pragma unroll
-          for (int u = 0; u < CPL; ++u)
-            if (u == nu) xn = r[u];
-          argmax_merge(bv, bi, abs1(xn), gi);
-        }
-      }
-    }
-  }
-
-  // ---- write the factored panel back ----
-#pragma unroll
-  for (int u = 0; u < CPL; ++u) {
-    const int c = phase + u * NCPH;
-    if (has_row && c < kb) A[(std::size_t)(k + c) * lda + (k + gi)] = r[u];
-  }
-  __syncthreads();
-  panel_finish(cluster, rank, k, kb, plist, flags, reinterpret_cast<int *>(smem_raw + o.map_pos),
-               reinterpret_cast<int *>(smem_raw + o.map_org), ipiv, perm, g_map_pos, g_map_src,
-               g_map_count, info);
-}
-
 // Load the kb x kb diagonal block A[k:k+kb, k:k+kb] into shared memory (D[l kb + i]
 // = A(k + i, k + l)): a warp per column, 16-byte copies when every column of
 // the block starts 16-byte aligned, else one element per copy. (The per-element
@@ -830,435 +614,30 @@ __global__ void __launch_bounds__(256)
     if (lane + 32 * v < kb) col[lane + 32 * v] = x[v];
 }
 
-// ---------------------------------------------------------------------------
-// One-CTA panel, two levels: the h x kb panel (kb <= 64) stays in global
-// memory (L2) and is factored in sub-panels of KBS columns; a sub-panel's rows
-// live in registers (thread t keeps rows t, t + NT, ... -- RPT of them), so a
-// pivot column costs one CTA-wide argmax and one or two barriers, with no cluster
-// barrier and no distributed shared memory. After each sub-panel the CTA
-// applies its swaps to the panel's other columns, solves the sub-panel's
-// U12 rows with the unit-lower L11, and updates the rest of the panel.
-// ---------------------------------------------------------------------------
-constexpr int kCtaChunk = 8;  // columns per register chunk of the in-panel update
+// Configurations of the one-row-per-thread panel: KB columns (a row's elements
+// in registers, the multipliers' KB columns in shared memory), at most MAXT
+// threads per CTA. Float and double and complex64 rows take 64 registers;
+// complex128 panels of up to 2048 rows run 32 columns (128 registers, 256
+// threads): 57 us against two times 27 us with 16 columns at 1024 rows, and half
+// as many swap and update launches between panels.
+template <typename T> struct RowsPanel;
+template <> struct RowsPanel<float> { static constexpr int KB = 64, MAXT = 512, KBs = 64, MAXTs = 512; };
+template <> struct RowsPanel<double> { static constexpr int KB = 32, MAXT = 512, KBs = 32, MAXTs = 512; };
+template <> struct RowsPanel<float2> { static constexpr int KB = 32, MAXT = 512, KBs = 32, MAXTs = 512; };
+template <> struct RowsPanel<double2> { static constexpr int KB = 16, MAXT = 512, KBs = 32, MAXTs = 256; };
+constexpr int kRowsMax = kPanelMaxCluster * 512;  // tallest panel of that kernel
+template <typename T> constexpr int short_rows() { return kPanelMaxCluster * RowsPanel<T>::MAXTs; }
 
-template <typename T>
-__device__ __forceinline__ void lds_vec8(const T *src, T (&dst)[kCtaChunk]) {
-  // 8 consecutive elements as 16-byte shared loads (src 16-byte aligned)
-  union {
-    float4 v[kCtaChunk * sizeof(T) / 16];
-    T e[kCtaChunk];
-  } u;
-  const float4 *s4 = reinterpret_cast<const float4 *>(src);
-#pragma unroll
-  for (int i = 0; i < (int)(kCtaChunk * sizeof(T) / 16); ++i) u.v[i] = s4[i];
-#pragma unroll
-  for (int i = 0; i < kCtaChunk; ++i) dst[i] = u.e[i];
-}
-
-// kRotate: the rotating-register column loop (measured faster for complex128
-// and float32 panels: C2 +3 %, C3 +4 %); otherwise the fully unrolled one
-// (faster for float64: the wider sub-panels make the rotation and the masked
-// update cost more than the smaller code saves).
-template <typename T> constexpr bool panel_rotates() {
-  return std::is_same<T, double2>::value || std::is_same<T, float>::value;
-}
-
-// One pivot step's search and row exchange. The pivot is the largest
-// |Re| + |Im| of column col among rows >= a, first index on ties; the owner of
-// row a publishes that row into slot kRowA (after the warps' slots). kOneBarrier: every warp's winner
-// publishes its whole row into the warp's slot before the single barrier, and
-// after it every thread agrees on the pivot p and reads the pivot row from its
-// slot (the caller alternates buffers by step: a slot is rewritten two steps
-// later, after every reader has passed the intervening barrier). Otherwise the
-// CTA argmax (one barrier) comes first and the pivot's owner alone publishes
-// its row into slot 0 before a second barrier; measured faster with one row
-// per thread (float64, 256 rows: 2.5 %), slower with two or more. Returns the
-// slot of the pivot row. forced: no comparable candidate (NaN column), p = a.
-template <typename T, int KBS, int RPT, bool kOneBarrier, int kRowA>
-__device__ __forceinline__ int panel_pivot(const T (&r)[RPT][KBS], int col, int a, int h, T (*wrow)[KBS],
-                                           unsigned long long *red_key, int *red_idx, int &p, bool &forced,
-                                           double &pv) {
-  const int tid = threadIdx.x, NT = blockDim.x;
-  double bv = -1.0;
-  int bi = INT_MAX;
-#pragma unroll
-  for (int q = 0; q < RPT; ++q) {
-    const int gi = tid + q * NT;
-    if (gi >= a && gi < h) argmax_merge(bv, bi, abs1(r[q][col]), gi);
-  }
-  if constexpr (kOneBarrier) {
-    const int lane = tid & 31, warp = tid >> 5;
-    const ArgMax wa = warp_argmax(argmax_key(bv, bi, bi != INT_MAX));
-#pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-      const int gi = tid + q * NT;
-      if (gi == a) {
-#pragma unroll
-        for (int c = 0; c < KBS; ++c) wrow[kRowA][c] = r[q][c];
-      }
-      if (gi == wa.idx) {
-#pragma unroll
-        for (int c = 0; c < KBS; ++c) wrow[warp][c] = r[q][c];
-      }
-    }
-    if (lane == 0) {
-      red_key[warp] = wa.key;
-      red_idx[warp] = wa.idx;
-    }
-    __syncthreads();
-    int wp;
-    const ArgMax am = cta_argmax_collect_at(red_key, red_idx, wp);
-    pv = __longlong_as_double((long long)am.key);
-    p = am.idx;
-    forced = false;
-    if (p >= h || p < a) {
-      p = a;
-      pv = 0.0;
-      forced = true;
-    }
-    return forced ? kRowA : wp;
-  } else {
-    const ArgMax am = cta_argmax(argmax_key(bv, bi, bi != INT_MAX), red_key, red_idx);
-    pv = __longlong_as_double((long long)am.key);
-    p = am.idx;
-    forced = false;
-    if (p >= h || p < a) {
-      p = a;
-      pv = 0.0;
-      forced = true;
-    }
-#pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-      const int gi = tid + q * NT;
-      if (gi == a) {
-#pragma unroll
-        for (int c = 0; c < KBS; ++c) wrow[kRowA][c] = r[q][c];
-      }
-      if (gi == p) {
-#pragma unroll
-        for (int c = 0; c < KBS; ++c) wrow[0][c] = r[q][c];
-      }
-    }
-    __syncthreads();
-    return 0;
-  }
-}
-
-template <typename T, int KBS, int RPT, int MAXT = 512, bool kRotate = panel_rotates<T>()>
-__global__ void __launch_bounds__(MAXT, 1)
-    lu_panel_cta_kernel(int n, T *__restrict__ A, int lda, int k, int kb, int *__restrict__ ipiv,
-                        int *__restrict__ perm, int *__restrict__ g_map_pos, int *__restrict__ g_map_src,
-                        int *__restrict__ g_map_count, int *__restrict__ info) {
-  cg::cluster_group cluster = cg::this_cluster();  // launched as a cluster of one
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int NT = blockDim.x, nwarps = NT >> 5;
-  const int h = n - k;
-  T *P = A + (std::size_t)k * lda + k;  // the panel: P[c * lda + i], i < h, c < kb
-  // per pivot step, alternating: slots 0..kW-1 each warp winner's row, slot
-  // kW row a before the exchange
-  constexpr int kW = MAXT / 32;  // warps at most (MAXT threads)
-  __shared__ __align__(16) T wrow[2][kW + 1][KBS];
-  __shared__ T l11[KBS][KBS + 1];
-  __shared__ __align__(16) T u12[KBS][kMaxKb];
-  __shared__ unsigned long long red_key[2][kW];
-  __shared__ int red_idx[2][kW];
-  __shared__ int plist[kMaxKb];
-  __shared__ int flags[1];
-  __shared__ int mpos[2 * kMaxKb], morg[2 * kMaxKb];
-  __shared__ int src_top[KBS], disp_row[KBS], disp_src[KBS], ndisp[1];
-
-  if (tid == 0) flags[0] = -1;
-  T r[RPT][KBS];
-  for (int sb = 0; sb < kb; sb += KBS) {
-    const int w = min(KBS, kb - sb);
-#pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-      const int gi = tid + q * NT;
-#pragma unroll
-      for (int c = 0; c < KBS; ++c)
-        r[q][c] = (gi >= sb && gi < h && c < w) ? P[(std::size_t)(sb + c) * lda + gi] : elem<T>::zero();
-    }
-    if constexpr (kRotate) {
-    // ---- factor the sub-panel, one pivot column at a time. Each row's
-    // registers rotate one place left after every step, so the pivot column
-    // is always r[q][0] and every step runs the same (rolled) code with
-    // static register indices; finished columns ride at the back of the row
-    // (still swapped with it) and the update is masked to the unfinished
-    // positions. After KBS steps (idle ones past w) the row is back in
-    // column order. ----
-#pragma unroll 1
-    for (int j = 0; j < KBS; ++j) {
-      if (j < w) {
-        const int a = sb + j, buf = j & 1;
-        int p;
-        bool forced;
-        double pv;
-        const int ps = panel_pivot<T, KBS, RPT, (RPT > 1), kW>(r, 0, a, h, wrow[buf], red_key[buf], red_idx[buf], p, forced, pv);
-        const T *prow = wrow[buf][ps];
-        if (tid == 0) {
-          plist[a] = p;
-          if (pv == 0.0 && flags[0] < 0) flags[0] = a;
-        }
-        const T piv = prow[0];
-        const bool singular = forced || is_zero(piv);
-        const bool use_recip = abs1(piv) >= safe_min<T>();
-        const T rpiv = singular ? elem<T>::one() : divide(elem<T>::one(), piv);
-        const int lim = w - j;  // positions 1 .. lim-1 hold unfinished columns
-#pragma unroll
-        for (int q = 0; q < RPT; ++q) {
-          const int gi = tid + q * NT;
-          if (gi < a || gi >= h) continue;
-          if (gi == a) {
-            if (p != a) {
-#pragma unroll
-              for (int c = 0; c < KBS; ++c) r[q][c] = prow[c];
-            }
-            continue;
-          }
-          if (gi == p) {
-#pragma unroll
-            for (int c = 0; c < KBS; ++c) r[q][c] = wrow[buf][kW][c];
-          }
-          const T l = singular ? r[q][0] : (use_recip ? mul(r[q][0], rpiv) : divide(r[q][0], piv));
-          r[q][0] = l;
-#pragma unroll
-          for (int c = 1; c < KBS; ++c)
-            if (c < lim) r[q][c] = sub(r[q][c], mul(l, prow[c]));
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < RPT; ++q) {
-        const T t0 = r[q][0];
-#pragma unroll
-        for (int c = 0; c + 1 < KBS; ++c) r[q][c] = r[q][c + 1];
-        r[q][KBS - 1] = t0;
-      }
-    }
-    } else {
-    // ---- factor the sub-panel, one pivot column at a time ----
-#pragma unroll
-    for (int j = 0; j < KBS; ++j) {
-      if (j >= w) break;
-      const int a = sb + j, buf = j & 1;
-      int p;
-      bool forced;
-      double pv;
-      const int ps = panel_pivot<T, KBS, RPT, (RPT > 1), kW>(r, j, a, h, wrow[buf], red_key[buf], red_idx[buf], p, forced, pv);
-      const T *prow = wrow[buf][ps];
-      if (tid == 0) {
-        plist[a] = p;
-        if (pv == 0.0 && flags[0] < 0) flags[0] = a;
-      }
-      const T piv = prow[j];
-      const bool singular = forced || is_zero(piv);
-      const bool use_recip = abs1(piv) >= safe_min<T>();
-      const T rpiv = singular ? elem<T>::one() : divide(elem<T>::one(), piv);
-#pragma unroll
-      for (int q = 0; q < RPT; ++q) {
-        const int gi = tid + q * NT;
-        if (gi < a || gi >= h) continue;
-        if (gi == a) {
-          if (p != a) {
-#pragma unroll
-            for (int c = 0; c < KBS; ++c) r[q][c] = prow[c];
-          }
-          continue;
-        }
-        if (gi == p) {
-#pragma unroll
-          for (int c = 0; c < KBS; ++c) r[q][c] = wrow[buf][kW][c];
-        }
-        const T l = singular ? r[q][j] : (use_recip ? mul(r[q][j], rpiv) : divide(r[q][j], piv));
-        r[q][j] = l;
-#pragma unroll
-        for (int c = j + 1; c < KBS; ++c)
-          if (c < w) r[q][c] = sub(r[q][c], mul(l, prow[c]));
-      }
-    }
-    }
-    // ---- sub-panel back to memory, L11 to shared memory ----
-#pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-      const int gi = tid + q * NT;
-      if (gi >= sb && gi < h) {
-#pragma unroll
-        for (int c = 0; c < KBS; ++c)
-          if (c < w) P[(std::size_t)(sb + c) * lda + gi] = r[q][c];
-      }
-      if (gi >= sb && gi < sb + w) {
-#pragma unroll
-        for (int c = 0; c < KBS; ++c) l11[gi - sb][c] = r[q][c];
-      }
-    }
-    // ---- where the sub-panel's swaps moved rows: position sb + j now holds
-    // old row src_top[j]; a row d below the block holds old top-block row
-    // disp_src[e] (rows below only ever receive rows of the top block) ----
-    // (every lane follows one final position back through the swaps, in
-    // reverse order, to the row it came from)
-    if (warp == 0) {
-      const int e = lane;
-      int x = -1;
-      if (e < w) x = sb + e;                                                      // a top-block position
-      else if (e < 2 * w && plist[sb + e - w] >= sb + w) x = plist[sb + e - w];  // a displaced row
-      if (x >= 0) {
-        const int fin = x;
-        for (int j = w - 1; j >= 0; --j) {
-          const int pj = plist[sb + j];
-          if (x == sb + j) x = pj;
-          else if (x == pj) x = sb + j;
-        }
-        if (e < w) src_top[e] = x;
-        else {
-          disp_row[e - w] = fin;
-          disp_src[e - w] = x;
-        }
-      } else if (e >= w && e < 2 * w) {
-        disp_row[e - w] = -1;
-      }
-      if (lane == 0) ndisp[0] = w;
-    }
-    __syncthreads();
-    // ---- the panel's other columns: swap, and right of the sub-panel solve
-    // the top block with L11 (U12 rows into shared memory) ----
-    if (tid < kb - w) {
-      const int c = tid < sb ? tid : tid + w;
-      T *col = P + (std::size_t)c * lda;
-      T top[KBS], x[KBS];
-#pragma unroll
-      for (int j = 0; j < KBS; ++j) top[j] = j < w ? col[sb + j] : elem<T>::zero();
-#pragma unroll
-      for (int j = 0; j < KBS; ++j) {
-        x[j] = elem<T>::zero();
-        if (j < w) {
-          const int src = src_top[j];
-          if (src >= sb + w) x[j] = col[src];
-          else {
-#pragma unroll
-            for (int q = 0; q < KBS; ++q)
-              if (q == src - sb) x[j] = top[q];
-          }
-        }
-      }
-      for (int e = 0; e < ndisp[0]; ++e) {
-        if (disp_row[e] < 0) continue;
-        const int srcq = disp_src[e] - sb;
-        T v = elem<T>::zero();
-#pragma unroll
-        for (int q = 0; q < KBS; ++q)
-          if (q == srcq) v = top[q];
-        col[disp_row[e]] = v;
-      }
-      if (c >= sb + w) {
-#pragma unroll
-        for (int j = 1; j < KBS; ++j)
-#pragma unroll
-          for (int q = 0; q < j; ++q)
-            if (j < w) x[j] = sub(x[j], mul(l11[j][q], x[q]));
-#pragma unroll
-        for (int j = 0; j < KBS; ++j)
-          if (j < w) u12[j][c] = x[j];
-      }
-#pragma unroll
-      for (int j = 0; j < KBS; ++j)
-        if (j < w) col[sb + j] = x[j];
-    }
-    __syncthreads();
-    // ---- update the rest of the panel: rows below the block, columns right
-    // of the sub-panel (the multipliers are reloaded from the written-back
-    // sub-panel, so no panel registers stay live through the column phase) ----
-    const int c0 = sb + w;
-    if (c0 < kb) {
-#pragma unroll
-      for (int q = 0; q < RPT; ++q) {
-        const int gi = tid + q * NT;
-        if (gi < c0 || gi >= h) continue;
-#pragma unroll
-        for (int j = 0; j < KBS; ++j) r[q][j] = j < w ? P[(std::size_t)(sb + j) * lda + gi] : elem<T>::zero();
-        for (int c = c0; c < kb; c += kCtaChunk) {
-          T v[kCtaChunk];
-#pragma unroll
-          for (int u = 0; u < kCtaChunk; ++u)
-            v[u] = c + u < kb ? P[(std::size_t)(c + u) * lda + gi] : elem<T>::zero();
-#pragma unroll
-          for (int j = 0; j < KBS; ++j) {
-            T b[kCtaChunk];
-            lds_vec8(&u12[j][c], b);
-#pragma unroll
-            for (int u = 0; u < kCtaChunk; ++u) v[u] = sub(v[u], mul(r[q][j], b[u]));
-          }
-#pragma unroll
-          for (int u = 0; u < kCtaChunk; ++u)
-            if (c + u < kb) P[(std::size_t)(c + u) * lda + gi] = v[u];
-        }
-      }
-    }
-    __syncthreads();
-  }
-  panel_finish(cluster, 0, k, kb, plist, flags, mpos, morg, ipiv, perm, g_map_pos, g_map_src, g_map_count,
-               info);
-}
-
-// One-CTA panel configurations by height: RPT rows per thread for heights up
-// to 512 RPT (512 threads), sub-panel width KBS (64 registers of sub-panel per
-// thread at most), outer panel width KB. Heights 2049..4096 take RPT8 rows per
-// thread on NT8 threads: float32 runs 1024 threads of 4 rows there (64
-// registers, a few spilled), measured 5 % faster on the float32 4096 expm than
-// 512 threads of 8 rows; float64 1024 x 2 rows at heights up to 2048, and
-// complex128 1024 x 1 row (sub-panels of 4) at 1024, measured slower. Panels
-// of 16 columns for float32, float64 and complex128: with the expm's launches
-// replayed as a graph, more and narrower panels cost less than a second
-// sub-panel's rest-of-panel update on the one SM (float64 256 expm +15 %,
-// complex128 1024 +4 %, float32 4096 +3 %; 8 columns: float32 4096 -20 %).
-template <typename T> struct CtaPanel;
-template <> struct CtaPanel<double2> {
-  static constexpr int KBS1 = 8, KBS2 = 8, KBS4 = 4, KBS8 = 0, RPT8 = 8, NT8 = 512, KB = 16;
-};
-template <> struct CtaPanel<double> {
-  static constexpr int KBS1 = 16, KBS2 = 16, KBS4 = 8, KBS8 = 4, RPT8 = 8, NT8 = 512, KB = 16;
-};
-template <> struct CtaPanel<float2> {
-  static constexpr int KBS1 = 16, KBS2 = 16, KBS4 = 8, KBS8 = 4, RPT8 = 8, NT8 = 512, KB = 32;
-};
-template <> struct CtaPanel<float> {  // 32 wide: the in-panel SIMT update costs h kb^2 / 2 per panel
-  static constexpr int KBS1 = 16, KBS2 = 16, KBS4 = 16, KBS8 = 8, RPT8 = 4, NT8 = 1024, KB = 16;
-};
-
-// Panel width of the one-CTA path for an n x n factorisation, 0 if n is too
-// tall for it.
-template <typename T>
-int cta_panel_kb(int n) {
-  const int kbs = n <= 512 ? CtaPanel<T>::KBS1 : n <= 1024 ? CtaPanel<T>::KBS2
-                : n <= 2048 ? CtaPanel<T>::KBS4 : n <= 4096 ? CtaPanel<T>::KBS8 : 0;
-  return kbs > 0 ? CtaPanel<T>::KB : 0;
-}
-
-// Register-panel configurations: KB columns, NCPH lanes per row, NT threads
-// per CTA (so NT / NCPH rows per CTA). Each lane keeps KB / NCPH elements,
-// 64 (RegPanel) or 128 (RegPanelWide, more rows per CTA) 32-bit registers.
-template <typename T> struct RegPanel;
-template <> struct RegPanel<double2> { static constexpr int KB = 32, NCPH = 4, NT = 512, kRows = NT / NCPH; };
-template <> struct RegPanel<double> { static constexpr int KB = 64, NCPH = 4, NT = 512, kRows = NT / NCPH; };
-template <> struct RegPanel<float2> { static constexpr int KB = 64, NCPH = 4, NT = 512, kRows = NT / NCPH; };
-template <> struct RegPanel<float> { static constexpr int KB = 64, NCPH = 2, NT = 512, kRows = NT / NCPH; };
-template <typename T> struct RegPanelWide;
-template <> struct RegPanelWide<double2> { static constexpr int KB = 32, NCPH = 1, NT = 256, kRows = NT / NCPH; };
-template <> struct RegPanelWide<double> { static constexpr int KB = 64, NCPH = 1, NT = 256, kRows = NT / NCPH; };
-template <> struct RegPanelWide<float2> { static constexpr int KB = 64, NCPH = 1, NT = 256, kRows = NT / NCPH; };
-template <> struct RegPanelWide<float> { static constexpr int KB = 64, NCPH = 1, NT = 512, kRows = NT / NCPH; };
-
-// Panel width of the outer blocking: complex128 panels are 32 wide so a row's
-// register share stays at 64 registers.
-template <typename T> constexpr int panel_width() { return RegPanel<T>::KB; }
-
-// Panel width for an n x n factorisation: the widest kb <= 64 whose full-height
-// panel fits in kMaxCluster CTAs' shared memory.
+// Panel width for an n x n factorisation: that of the one-row-per-thread
+// panel; beyond its tallest panel, the widest whose full-height panel fits in
+// kMaxCluster CTAs' shared memory (lu_panel_kernel).
 template <typename T>
 int choose_kb(int n) {
-  int kb = panel_width<T>();
-  while (kb > 1 && (std::size_t)n * kb * sizeof(T) > kPanelSmemBudget * kMaxCluster) kb /= 2;
+  if (n <= short_rows<T>()) return RowsPanel<T>::KBs;
+  int kb = RowsPanel<T>::KB;
+  while (kb > 1 && n > kRowsMax && (std::size_t)n * kb * sizeof(T) > kPanelSmemBudget * kMaxCluster) kb /= 2;
   return kb;
 }
-
 
 inline cudaLaunchAttribute cluster_attr(int ncta) {
   cudaLaunchAttribute a;
@@ -1269,80 +648,41 @@ inline cudaLaunchAttribute cluster_attr(int ncta) {
   return a;
 }
 
-template <typename T, int KB, int NCPH, int NT>
-cudaError_t launch_reg_panel(cudaStream_t s, int n, T *A, int lda, int k, int kb, const LuScratch &sc,
-                             int *info) {
-  constexpr int kRows = NT / NCPH;
+// One row per thread: one CTA up to 512 rows, where the exchange between CTAs
+// costs more than the warps that share an SM (a float64 column of 512 rows:
+// 1.09 us in one CTA, 1.22 to 1.28 in 2 to 8); above, always eight CTAs, since
+// fewer rows per SM shorten the update (float64, 2048 rows: 1.54 us a column on
+// four CTAs, 1.37 on eight).
+template <typename T, int KB, int MAXT>
+cudaError_t launch_rows_panel(cudaStream_t s, int n, T *A, int lda, int k, int kb, const LuScratch &sc, int *info) {
   const int h = n - k;
-  const int ncta = (h + kRows - 1) / kRows;
-  const int rpc = (h + ncta - 1) / ncta;
-  const PanelSmem o = panel_smem<T>(0, KB);
-  auto kern = lu_panel_reg_kernel<T, KB, NCPH, NT>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)o.total);
+  const int ncta = h <= MAXT ? 1 : kPanelMaxCluster;
+  int nt = ((h + ncta - 1) / ncta + 31) / 32 * 32;
+  if (nt < 64) nt = 64;  // the threads that list the rows moved down: kb <= 64
+  auto kern = lu_panel_rows_kernel<T, KB, MAXT>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)panel_rows_smem<T, KB>(MAXT));
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ncta, 1, 1);
-  int nt = ((rpc * NCPH + 31) / 32) * 32;
-  if (nt < 64) nt = 64;
   cfg.blockDim = dim3(nt, 1, 1);
-  cfg.dynamicSmemBytes = o.total;
+  cfg.dynamicSmemBytes = panel_rows_smem<T, KB>(nt);
   cfg.stream = s;
   cudaLaunchAttribute attr[1] = {cluster_attr(ncta)};
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   note_launch();
-  return cudaLaunchKernelEx(&cfg, kern, n, A, lda, k, kb, rpc, sc.ipiv, sc.perm, sc.map_pos,
-                            sc.map_src, sc.map_count, info);
-}
-
-template <typename T, int KBS, int RPT, int MAXT = 512>
-cudaError_t launch_cta_panel_cfg(cudaStream_t s, int n, T *A, int lda, int k, int kb, const LuScratch &sc,
-                                 int *info) {
-  const int h = n - k;
-  int nt = (h + RPT - 1) / RPT;
-  nt = ((nt + 31) / 32) * 32;
-  if (nt < 64) nt = 64;  // >= kb - KBS column threads
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(1, 1, 1);
-  cfg.blockDim = dim3(nt, 1, 1);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1] = {cluster_attr(1)};
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  note_launch();
-  return cudaLaunchKernelEx(&cfg, lu_panel_cta_kernel<T, KBS, RPT, MAXT>, n, A, lda, k, kb, sc.ipiv, sc.perm,
-                            sc.map_pos, sc.map_src, sc.map_count, info);
-}
-
-// The one-CTA panel for a step of an n x n factorisation (kb = cta_panel_kb).
-template <typename T>
-cudaError_t launch_cta_panel(cudaStream_t s, int n, T *A, int lda, int k, int kb, const LuScratch &sc,
-                             int *info) {
-  using C = CtaPanel<T>;
-  if (n <= 512) {
-    if constexpr (C::KBS1 > 0) return launch_cta_panel_cfg<T, C::KBS1, 1>(s, n, A, lda, k, kb, sc, info);
-  } else if (n <= 1024) {
-    if constexpr (C::KBS2 > 0) return launch_cta_panel_cfg<T, C::KBS2, 2>(s, n, A, lda, k, kb, sc, info);
-  } else if (n <= 2048) {
-    if constexpr (C::KBS4 > 0) return launch_cta_panel_cfg<T, C::KBS4, 4>(s, n, A, lda, k, kb, sc, info);
-  } else {
-    if constexpr (C::KBS8 > 0)
-      return launch_cta_panel_cfg<T, C::KBS8, C::RPT8, C::NT8>(s, n, A, lda, k, kb, sc, info);
-  }
-  return cudaErrorInvalidValue;
+  return cudaLaunchKernelEx(&cfg, kern, n, A, lda, k, kb, sc.ipiv, sc.perm, sc.map_pos, sc.map_src, sc.map_count,
+                            info);
 }
 
 template <typename T>
 cudaError_t launch_panel(cudaStream_t s, int n, T *A, int lda, int k, int kb, const LuScratch &sc,
                          int *info) {
   const int h = n - k;
-  if (kb <= RegPanel<T>::KB && h <= kMaxCluster * RegPanel<T>::kRows) {
-    return launch_reg_panel<T, RegPanel<T>::KB, RegPanel<T>::NCPH, RegPanel<T>::NT>(s, n, A, lda, k, kb, sc, info);
-  }
-  if (kb <= RegPanel<T>::KB && h <= kMaxCluster * RegPanelWide<T>::kRows) {
-    return launch_reg_panel<T, RegPanelWide<T>::KB, RegPanelWide<T>::NCPH, RegPanelWide<T>::NT>(s, n, A, lda, k, kb, sc, info);
-  }
+  using C = RowsPanel<T>;
+  if (n <= short_rows<T>()) return launch_rows_panel<T, C::KBs, C::MAXTs>(s, n, A, lda, k, kb, sc, info);
+  if (h <= kRowsMax) return launch_rows_panel<T, C::KB, C::MAXT>(s, n, A, lda, k, kb, sc, info);
   // enough CTAs for the panel to fit, and for every row to get >= 2 lanes of
   // the fused pass when the cluster allows it (<= 256 rows per CTA)
   int ncta = (int)(((std::size_t)h * kb * sizeof(T) + kPanelSmemBudget - 1) / kPanelSmemBudget);
@@ -1439,8 +779,7 @@ cudaError_t getrf(cudaStream_t s, int n, T *A, int lda, void *scratch, int *info
   if (e != cudaSuccess) return e;
   iota_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, sc.perm);
   if ((e = launched()) != cudaSuccess) return e;
-  const int kb_cta = cta_panel_kb<T>(n);
-  const int kbn = kb_cta > 0 ? kb_cta : choose_kb<T>(n);
+  const int kbn = choose_kb<T>(n);
   auto swap_kern = lu_swap_trsm_kernel<T>;
   const std::size_t swap_smem = sizeof(T) * (std::size_t)kbn * kbn;
   if ((e = cudaFuncSetAttribute(swap_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)swap_smem)) !=
@@ -1452,8 +791,7 @@ cudaError_t getrf(cudaStream_t s, int n, T *A, int lda, void *scratch, int *info
   LookAhead *la = nullptr;
   if (ahead && (e = lookahead(la)) != cudaSuccess) return e;
   auto panel = [&](cudaStream_t st, int k, int kb) {
-    return kb_cta > 0 ? launch_cta_panel<T>(st, n, A, lda, k, kb, sc, info_dev)
-                      : launch_panel<T>(st, n, A, lda, k, kb, sc, info_dev);
+    return launch_panel<T>(st, n, A, lda, k, kb, sc, info_dev);
   };
   if ((e = panel(s, 0, kbn < n ? kbn : n)) != cudaSuccess) return e;
   for (int k = 0; k < n; k += kbn) {

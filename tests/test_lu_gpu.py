@@ -138,3 +138,63 @@ def test_pade_large_norm_pivoting(oracle, suf, m, target, cuda):
     run.close()
     assert st.ok and list(info) == [0, 0]
     assert rel_frob(r, ref) <= (1e-11 if suf in "dz" else 1e-3)
+
+
+def hadamard(n):
+    h = np.ones((1, 1))
+    while h.shape[0] < n:
+        h = np.block([[h, h], [h, -h]])
+    return h
+
+
+@pytest.mark.parametrize("suf", ["s", "d", "c", "z"])
+@pytest.mark.parametrize("n", [64, 512, 1024])  # one CTA, its largest height, a cluster of eight
+def test_getrf_ties_take_the_first_row(lib, oracle, suf, n):
+    """A Hadamard matrix eliminates without rounding (entries stay powers of two) and ties in every
+    column: the pivots are IxAMAX's, and the factors are exact."""
+    a = hadamard(n).astype(NP_DTYPE[suf])
+    _, _, lu, ipiv, info = run_getrf(lib, a, suf)
+    olu, opiv, oinfo = oracle.getrf(a.astype(np.complex128 if suf in "cz" else np.float64))
+    assert info == oinfo == 0
+    assert np.array_equal(ipiv, opiv)
+    assert np.array_equal(lu, olu.astype(lu.dtype))
+
+
+@pytest.mark.parametrize("suf,n", [("d", 33), ("d", 511), ("z", 31), ("z", 257), ("d", 2049)])
+def test_getrf_panel_edges(lib, oracle, suf, n):
+    """Ragged last panels and the heights next to a change of the panel's cluster."""
+    a = gaussian(n, suf, 910 + n)
+    _, _, lu, ipiv, info = run_getrf(lib, a, suf)
+    olu, opiv, oinfo = oracle.getrf(a)
+    assert info == oinfo == 0 and np.array_equal(ipiv, opiv)
+    assert np.abs(lu - olu).max() <= 1e-12 * max(1.0, np.abs(olu).max()) * np.sqrt(n)
+
+
+@pytest.mark.parametrize("suf,n", [("s", 4096), ("s", 4097), ("z", 2049), ("c", 2300)])
+def test_getrf_tallest_panels(lib, suf, n):
+    """The tallest one-row-per-thread panels and the first size beyond them, by their residual:
+    |PA - LU| <= n eps |L||U| element by element, |L| <= sqrt(2), |U| measured."""
+    import torch
+
+    a = gaussian(n, suf, 920 + n)
+    _, _, lu, ipiv, info = run_getrf(lib, a, suf)
+    assert info == 0
+    t = torch.from_numpy(lu.astype(np.complex128 if suf in "cz" else np.float64)).cuda()
+    L, U = torch.tril(t, -1), torch.triu(t)
+    L.diagonal().fill_(1.0)
+    perm = np.arange(n)
+    for j, p in enumerate(ipiv):
+        perm[[j, p]] = perm[[p, j]]
+    pa = torch.from_numpy(a.astype(np.complex128 if suf in "cz" else np.float64)[perm]).cuda()
+    assert bool(((pa - L @ U).abs() <= n * eps(suf) * (L.abs() @ U.abs())).all())
+    assert float(torch.tril(t, -1).abs().max()) <= (np.sqrt(2.0) if suf in "cz" else 1.0) * (1 + 1e-6)
+
+
+@pytest.mark.parametrize("n", [96, 700])
+def test_getrf_nan_column_keeps_its_row(lib, oracle, n):
+    """A column of NaNs has no candidate: its own row is kept, as the oracle does."""
+    a = gaussian(n, "d", 930 + n)
+    a[:, 40] = np.nan
+    _, _, _, ipiv, info = run_getrf(lib, a, "d")
+    _, opiv, _ = oracle.getrf(a)
+    assert np.array_equal(ipiv[:41], opiv[:41]) and ipiv[40] == 40
