@@ -104,6 +104,24 @@ def run_tc_c(lib, a, b, c0, alpha, beta, terms, lda=None):
 
 
 @pytest.mark.parametrize("terms", [6, 3])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (127, 129, 7), (257, 64, 64), (130, 300, 65), (128, 128, 128)])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_few_k_blocks(lib, terms, m, n, k, cplx):
+    """Depths of one and two k-blocks (the split inside the GEMM), ragged in every dimension, with an old C."""
+    rng = np.random.default_rng(m + 5 * n + 11 * k)
+    dt = np.complex64 if cplx else np.float32
+    draw = lambda *sh: (rng.standard_normal(sh) + (1j * rng.standard_normal(sh) if cplx else 0)).astype(dt)
+    a, b, c = draw(m, k), draw(k, n), draw(m, n)
+    kk = k // 2 or 1 if cplx and k > 64 else k  # complex: a depth of 64 is two k-blocks of the real product
+    a, b = a[:, :kk], b[:kk]
+    got = (run_tc_c if cplx else run_tc)(lib, a, b, c, -1.0, 1.0, terms, lda=m + 3)
+    wide = np.complex128 if cplx else np.float64
+    ref = c.astype(wide) - a.astype(wide) @ b.astype(wide)
+    rel = np.linalg.norm(got - ref) / (np.linalg.norm(a) * np.linalg.norm(b) + np.linalg.norm(c))
+    assert rel <= BOUND[terms], rel
+
+
+@pytest.mark.parametrize("terms", [6, 3])
 @pytest.mark.parametrize("m,n,k", [(128, 128, 64), (100, 70, 33), (300, 260, 129), (512, 512, 512)])
 def test_complex64_split_gemm_matches_fp64(lib, terms, m, n, k):
     """complex64 as one real product of the block form [[Ar, -Ai]; [Ai, Ar]] [Br; Bi]"""
