@@ -126,8 +126,7 @@ calamanStatus_t pade_run(cudaStream_t st, int m, int n, const T *A, int lda, T *
   CLM_CUDA(mm(A, lda, ws.W, n, 0.0, U));  // U = A W
   // p = V + U over U (the same thread reads then writes each element), q = V - U over V
   CLM_CUDA(launch_pade_split<T>(st, n, U, ws.V, U, n, ws.V));
-  CLM_CUDA(getrf<T>(st, n, ws.V, n, ws.lu, d_info));
-  CLM_CUDA(getrs<T>(st, n, n, ws.V, n, ws.lu, U, n, R, ldr, d_info + 1));
+  CLM_CUDA(getrf_solve<T>(st, n, ws.V, n, ws.lu, n, U, n, R, ldr, false, d_info));
   return ok_status();
 }
 

@@ -118,6 +118,15 @@ template <typename T>
 cudaError_t getrs(cudaStream_t s, int n, int nrhs, const T *LU, int lda, const void *scratch,
                   const T *B, int ldb, T *X, int ldx, int *info_dev);
 
+// Both at once: factor A and solve A X = B for nrhs columns, the forward
+// substitution run beside the factorisation. B is overwritten; B and X may not
+// alias. keep_l: L is left as getrf leaves it (getrs may follow); otherwise its
+// rows are in the order of their own panel's factorisation. info_dev[0] as
+// getrf's, info_dev[1] as getrs's.
+template <typename T>
+cudaError_t getrf_solve(cudaStream_t s, int n, T *A, int lda, void *scratch, int nrhs, T *B, int ldb, T *X, int ldx,
+                        bool keep_l, int *info_dev);
+
 // B = f op(A) for an rows x cols matrix A: op is the transpose, conjugated
 // when `conj` (complex types); B is cols x rows. A and B may not alias.
 template <typename T>

@@ -42,18 +42,26 @@ constexpr int kPanelThreads = 512;
 constexpr int kMaxCluster = 8;
 constexpr std::size_t kPanelSmemBudget = 176 * 1024;  // bytes of panel per CTA
 
-// scratch: ipiv[n] | perm[n] | map_pos[2*kMaxKb] | map_src[2*kMaxKb] | map_count
+// scratch: ipiv[n] | perm[n] | two row maps (of even and of odd panels: a
+// panel's swaps are still replayed while the next panel writes its own), each
+// map_pos[2*kMaxKb] | map_src[2*kMaxKb] | map_count
+struct RowMap {
+  int *pos, *src, *count;
+};
 struct LuScratch {
-  int *ipiv, *perm, *map_pos, *map_src, *map_count;
+  int *ipiv, *perm;
+  RowMap map[2];
 };
 inline LuScratch carve_lu(void *base, int n) {
   Layout L(base);
   LuScratch s;
   s.ipiv = L.take<int>(n);
   s.perm = L.take<int>(n);
-  s.map_pos = L.take<int>(2 * kMaxKb);
-  s.map_src = L.take<int>(2 * kMaxKb);
-  s.map_count = L.take<int>(1);
+  for (RowMap &m : s.map) {
+    m.pos = L.take<int>(2 * kMaxKb);
+    m.src = L.take<int>(2 * kMaxKb);
+    m.count = L.take<int>(1);
+  }
   return s;
 }
 
@@ -438,10 +446,16 @@ __device__ __forceinline__ void load_diag_block(T *D, const T *A, int lda, int k
   cp_async_wait_all();
 }
 
-// ---- swap + TRSM for the columns outside the panel: one warp per column ----
+// ---- swap + TRSM of one panel for columns outside it: one warp per column ----
+// Columns [c0, c0 + nright) right of the panel, then nrhs columns of a right-
+// hand side B (both: swaps, then the solve with the unit-lower L11), then the
+// nleft first columns of A (swaps only). The solved rows of a right-hand side
+// go to rows k .. k + kb - 1 of X; the rows the swaps moved down stay in B,
+// whose rows below the panel are still being updated.
 template <typename T>
 __global__ void __launch_bounds__(256)
-    lu_swap_trsm_kernel(int n, T *__restrict__ A, int lda, int k, int kb,
+    lu_swap_trsm_kernel(T *__restrict__ A, int lda, int k, int kb, int c0, int nright, int nleft,
+                        T *__restrict__ B, int ldb, T *__restrict__ X, int ldx, int nrhs,
                         const int *__restrict__ map_pos, const int *__restrict__ map_src,
                         const int *__restrict__ map_count) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -449,12 +463,11 @@ __global__ void __launch_bounds__(256)
   const int warps = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   const int ci = blockIdx.x * warps + (threadIdx.x >> 5);
-  const bool block_needs_L = (int)(blockIdx.x + 1) * warps > k;  // holds a right-of-panel column
-  if (block_needs_L) load_diag_block(L, A, lda, k, kb);
+  if ((int)blockIdx.x * warps < nright + nrhs) load_diag_block(L, A, lda, k, kb);  // holds a column to solve
   __syncthreads();
-  if (ci >= n - kb) return;
-  const int c = ci < k ? ci : ci + kb;
-  T *col = A + (std::size_t)c * lda;
+  if (ci >= nright + nrhs + nleft) return;
+  const bool rhs = ci >= nright && ci < nright + nrhs, left = ci >= nright + nrhs;
+  T *col = rhs ? B + (std::size_t)(ci - nright) * ldb : A + (std::size_t)(left ? ci - nright - nrhs : c0 + ci) * lda;
   const int cnt = *map_count;
   T v[4];
 #pragma unroll
@@ -463,7 +476,7 @@ __global__ void __launch_bounds__(256)
     v[q] = e < cnt ? col[map_src[e]] : elem<T>::zero();
   }
   __syncwarp();
-  if (c < k) {
+  if (left) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int e = lane + 32 * q;
@@ -482,8 +495,9 @@ __global__ void __launch_bounds__(256)
     if (lane > l && lane < kb) x0 = sub(x0, mul(L[l * kb + lane], xl));
     if (lane + 32 > l && lane + 32 < kb) x1 = sub(x1, mul(L[l * kb + lane + 32], xl));
   }
-  if (lane < kb) col[k + lane] = x0;
-  if (lane + 32 < kb) col[k + lane + 32] = x1;
+  T *out = rhs ? X + (std::size_t)(ci - nright) * ldx : col;
+  if (lane < kb) out[k + lane] = x0;
+  if (lane + 32 < kb) out[k + lane + 32] = x1;
 }
 
 __global__ void iota_kernel(int n, int *p) {
@@ -654,7 +668,8 @@ inline cudaLaunchAttribute cluster_attr(int ncta) {
 // fewer rows per SM shorten the update (float64, 2048 rows: 1.54 us a column on
 // four CTAs, 1.37 on eight).
 template <typename T, int KB, int MAXT>
-cudaError_t launch_rows_panel(cudaStream_t s, int n, T *A, int lda, int k, int kb, const LuScratch &sc, int *info) {
+cudaError_t launch_rows_panel(cudaStream_t s, int n, T *A, int lda, int k, int kb, const LuScratch &sc,
+                              const RowMap &map, int *info) {
   const int h = n - k;
   const int ncta = h <= MAXT ? 1 : kPanelMaxCluster;
   int nt = ((h + ncta - 1) / ncta + 31) / 32 * 32;
@@ -672,17 +687,16 @@ cudaError_t launch_rows_panel(cudaStream_t s, int n, T *A, int lda, int k, int k
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   note_launch();
-  return cudaLaunchKernelEx(&cfg, kern, n, A, lda, k, kb, sc.ipiv, sc.perm, sc.map_pos, sc.map_src, sc.map_count,
-                            info);
+  return cudaLaunchKernelEx(&cfg, kern, n, A, lda, k, kb, sc.ipiv, sc.perm, map.pos, map.src, map.count, info);
 }
 
 template <typename T>
 cudaError_t launch_panel(cudaStream_t s, int n, T *A, int lda, int k, int kb, const LuScratch &sc,
-                         int *info) {
+                         const RowMap &map, int *info) {
   const int h = n - k;
   using C = RowsPanel<T>;
-  if (n <= short_rows<T>()) return launch_rows_panel<T, C::KBs, C::MAXTs>(s, n, A, lda, k, kb, sc, info);
-  if (h <= kRowsMax) return launch_rows_panel<T, C::KB, C::MAXT>(s, n, A, lda, k, kb, sc, info);
+  if (n <= short_rows<T>()) return launch_rows_panel<T, C::KBs, C::MAXTs>(s, n, A, lda, k, kb, sc, map, info);
+  if (h <= kRowsMax) return launch_rows_panel<T, C::KB, C::MAXT>(s, n, A, lda, k, kb, sc, map, info);
   // enough CTAs for the panel to fit, and for every row to get >= 2 lanes of
   // the fused pass when the cluster allows it (<= 256 rows per CTA)
   int ncta = (int)(((std::size_t)h * kb * sizeof(T) + kPanelSmemBudget - 1) / kPanelSmemBudget);
@@ -715,8 +729,8 @@ cudaError_t launch_panel(cudaStream_t s, int n, T *A, int lda, int k, int kb, co
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   note_launch();
-  return cudaLaunchKernelEx(&cfg, kern, n, A, lda, k, kb, rpc, sc.ipiv, sc.perm, sc.map_pos,
-                            sc.map_src, sc.map_count, info);
+  return cudaLaunchKernelEx(&cfg, kern, n, A, lda, k, kb, rpc, sc.ipiv, sc.perm, map.pos, map.src, map.count,
+                            info);
 }
 
 }  // namespace
@@ -725,9 +739,11 @@ std::size_t lu_scratch_bytes(int n) {
   Layout L(nullptr);
   L.take<int>(n < 1 ? 1 : n);  // ipiv
   L.take<int>(n < 1 ? 1 : n);  // perm
-  L.take<int>(2 * kMaxKb);     // map_pos
-  L.take<int>(2 * kMaxKb);     // map_src
-  L.take<int>(1);              // map_count
+  for (int i = 0; i < 2; ++i) {  // the row maps
+    L.take<int>(2 * kMaxKb);
+    L.take<int>(2 * kMaxKb);
+    L.take<int>(1);
+  }
   return L.used;
 }
 
@@ -766,15 +782,21 @@ cudaError_t lookahead(LookAhead *&out) {
   return cudaSuccess;
 }
 
-// Blocked right-looking factorisation with a one-panel look-ahead: after the
-// swaps and U12 solve of panel k, the next panel's columns are updated first
-// (a narrow GEMM); panel k+1 is then factored on the auxiliary stream while
-// the caller's stream updates the columns beyond it, and panel k+1's swaps wait
-// for both.
+// Blocked right-looking factorisation with a one-panel look-ahead. The panel
+// is a latency chain on at most eight SMs, so what it waits for comes first:
+// after panel k, the swaps, U12 and the update of the next panel's columns
+// alone; then panel k+1 runs on the auxiliary stream while the caller's stream
+// does the same for the other columns. With a right-hand side (B != null) its
+// forward substitution is part of that: B's columns take the swaps, the solve
+// with L11 and the update like the matrix's own, in the time that the caller's
+// stream would wait for the panels, and X receives L^-1 P B; B is overwritten.
+// The columns left of a panel take its swaps (keep_l) only where L is used
+// again. Forward substitution after the factorisation, against this: complex128
+// 1024 expm 4986 -> 4638 us, float64 1501 5555 -> 5035, float32 4096 15478 ->
+// 12918 (with the split inside its updates), complex64 777 3123 -> 2591.
 template <typename T>
-cudaError_t getrf(cudaStream_t s, int n, T *A, int lda, void *scratch, int *info_dev) {
-  if (n < 1) return cudaSuccess;
-  const LuScratch sc = carve_lu(scratch, n);
+static cudaError_t factor(cudaStream_t s, int n, T *A, int lda, const LuScratch &sc, int *info_dev, bool keep_l,
+                          int nrhs, T *B, int ldb, T *X, int ldx) {
   cudaError_t e = cudaMemsetAsync(info_dev, 0, sizeof(int), s);
   if (e != cudaSuccess) return e;
   iota_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, sc.perm);
@@ -790,59 +812,63 @@ cudaError_t getrf(cudaStream_t s, int n, T *A, int lda, void *scratch, int *info
   const bool ahead = n > kbn && !tl_no_lookahead;
   LookAhead *la = nullptr;
   if (ahead && (e = lookahead(la)) != cudaSuccess) return e;
-  auto panel = [&](cudaStream_t st, int k, int kb) {
-    return launch_panel<T>(st, n, A, lda, k, kb, sc, info_dev);
-  };
-  if ((e = panel(s, 0, kbn < n ? kbn : n)) != cudaSuccess) return e;
-  for (int k = 0; k < n; k += kbn) {
+  if ((e = launch_panel<T>(s, n, A, lda, 0, kbn < n ? kbn : n, sc, sc.map[0], info_dev)) != cudaSuccess) return e;
+  for (int k = 0, step = 0; k < n; k += kbn, ++step) {
     const int kb = (k + kbn < n) ? kbn : n - k;
+    const RowMap &map = sc.map[step & 1];
     if (ahead && k > 0 && (e = cudaStreamWaitEvent(s, la->done, 0)) != cudaSuccess) return e;  // panel k
-    const int others = n - kb;
-    if (others > 0) {
+    // swaps and solve of nright columns from c0 on, of the right-hand side, and swaps of nleft columns
+    auto swaps = [&](int c0, int nright, int rhs, int nleft) -> cudaError_t {
+      const int cols = nright + rhs + nleft;
+      if (cols == 0) return cudaSuccess;
       const int warps = 8;
-      swap_kern<<<(others + warps - 1) / warps, warps * 32, sizeof(T) * (std::size_t)kb * kb, s>>>(
-          n, A, lda, k, kb, sc.map_pos, sc.map_src, sc.map_count);
-      if ((e = launched()) != cudaSuccess) return e;
-    }
+      swap_kern<<<(cols + warps - 1) / warps, warps * 32, sizeof(T) * (std::size_t)kb * kb, s>>>(
+          A, lda, k, kb, c0, nright, nleft, B, ldb, X, ldx, rhs, map.pos, map.src, map.count);
+      return launched();
+    };
     const int rest = n - (k + kb);
-    if (rest > 0) {
-      const int kb2 = rest < kbn ? rest : kbn;  // the next panel's width
-      const T *L21 = A + (std::size_t)k * lda + (k + kb);
-      // next panel's columns first
-      e = gemm_nn<T>(s, rest, kb2, kb, -1.0, L21, lda, A + (std::size_t)(k + kb) * lda + k, lda, 1.0,
-                     A + (std::size_t)(k + kb) * lda + (k + kb), lda);
-      if (e != cudaSuccess) return e;
+    const int kb2 = rest < kbn ? rest : kbn;  // the next panel's width
+    const T *L21 = A + (std::size_t)k * lda + (k + kb);
+    auto update = [&](const T *U, int ldu, T *C, int ldc, int cols) -> cudaError_t {
+      if (rest == 0 || cols == 0) return cudaSuccess;
+      return gemm_nn<T>(s, rest, cols, kb, -1.0, L21, lda, U, ldu, 1.0, C, ldc);
+    };
+    if (rest > 0) {  // the next panel's columns first
+      T *next = A + (std::size_t)(k + kb) * lda + k;
+      if ((e = swaps(k + kb, kb2, 0, 0)) != cudaSuccess) return e;
+      if ((e = update(next, lda, next + kb, lda, kb2)) != cudaSuccess) return e;
       if (ahead) {
         if ((e = cudaEventRecord(la->ready, s)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(la->aux, la->ready, 0)) != cudaSuccess) return e;
-        if ((e = panel(la->aux, k + kb, kb2)) != cudaSuccess) return e;
+        if ((e = launch_panel<T>(la->aux, n, A, lda, k + kb, kb2, sc, sc.map[(step + 1) & 1], info_dev)) != cudaSuccess)
+          return e;
         if ((e = cudaEventRecord(la->done, la->aux)) != cudaSuccess) return e;
-      } else if ((e = panel(s, k + kb, kb2)) != cudaSuccess) {  // disjoint from the wide update
+      } else if ((e = launch_panel<T>(s, n, A, lda, k + kb, kb2, sc, sc.map[(step + 1) & 1], info_dev)) !=
+                 cudaSuccess) {  // disjoint from the other columns
         return e;
       }
-      // the wide update, concurrent with that panel
-      if (rest > kb2) {
-        e = gemm_nn<T>(s, rest, rest - kb2, kb, -1.0, L21, lda, A + (std::size_t)(k + kb + kb2) * lda + k, lda,
-                       1.0, A + (std::size_t)(k + kb + kb2) * lda + (k + kb), lda);
-        if (e != cudaSuccess) return e;
-      }
     }
+    // the other columns, concurrent with that panel
+    const int c1 = k + kb + kb2;
+    if ((e = swaps(c1, n - c1, nrhs, keep_l ? k : 0)) != cudaSuccess) return e;
+    T *U = A + (std::size_t)c1 * lda + k;
+    if ((e = update(U, lda, U + kb, lda, n - c1)) != cudaSuccess) return e;
+    if (nrhs > 0 && (e = update(X + k, ldx, B + k + kb, ldb, nrhs)) != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
 
 template <typename T>
-cudaError_t getrs(cudaStream_t s, int n, int nrhs, const T *LU, int lda, const void *scratch,
-                  const T *B, int ldb, T *X, int ldx, int *info_dev) {
-  if (n < 1 || nrhs < 1) return cudaSuccess;
-  const LuScratch sc = carve_lu(const_cast<void *>(scratch), n);
-  cudaError_t e = cudaMemsetAsync(info_dev, 0, sizeof(int), s);
-  if (e != cudaSuccess) return e;
-  {
-    const int gy = nrhs < 65535 ? nrhs : 65535;
-    gather_rows_kernel<T><<<dim3((n + 255) / 256, gy), 256, 0, s>>>(n, nrhs, sc.perm, B, ldb, X, ldx);
-    if ((e = launched()) != cudaSuccess) return e;
-  }
+cudaError_t getrf(cudaStream_t s, int n, T *A, int lda, void *scratch, int *info_dev) {
+  if (n < 1) return cudaSuccess;
+  return factor<T>(s, n, A, lda, carve_lu(scratch, n), info_dev, true, 0, nullptr, 0, nullptr, 0);
+}
+
+// X <- L^-1 X (lower) and X <- U^-1 X (upper) by diagonal blocks.
+template <typename T>
+static cudaError_t triangular_solves(cudaStream_t s, int n, int nrhs, const T *LU, int lda, T *X, int ldx, bool lower,
+                                     bool upper) {
+  cudaError_t e;
   // Diagonal blocks of 64 rows; float32 systems above 1024 take 128 (half as
   // many passes of the off-diagonal updates over the right-hand side: float32
   // 4096 expm +3 %; float64 2048 measured 8 % slower with 128)
@@ -862,7 +888,7 @@ cudaError_t getrs(cudaStream_t s, int n, int nrhs, const T *LU, int lda, const v
     if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
       return e;
   const int blocks = (nrhs + warps - 1) / warps;
-  for (int k = 0; k < n; k += NB) {
+  for (int k = 0; lower && k < n; k += NB) {
     const int kb = (k + NB < n) ? NB : n - k;
     if (kb == NB) fl<<<blocks, warps * 32, sizeof(T) * (kb * kb + kb), s>>>(nrhs, LU, lda, k, X, ldx);
     else kl<<<blocks, warps * 32, sizeof(T) * (kb * kb + kb), s>>>(nrhs, LU, lda, k, kb, X, ldx);
@@ -874,7 +900,7 @@ cudaError_t getrs(cudaStream_t s, int n, int nrhs, const T *LU, int lda, const v
     }
   }
   const int last = ((n - 1) / NB) * NB;
-  for (int k = last; k >= 0; k -= NB) {
+  for (int k = last; upper && k >= 0; k -= NB) {
     const int kb = (k + NB < n) ? NB : n - k;
     if (kb == NB) fu<<<blocks, warps * 32, sizeof(T) * (kb * kb + kb), s>>>(nrhs, LU, lda, k, X, ldx);
     else ku<<<blocks, warps * 32, sizeof(T) * (kb * kb + kb), s>>>(nrhs, LU, lda, k, kb, X, ldx);
@@ -887,10 +913,37 @@ cudaError_t getrs(cudaStream_t s, int n, int nrhs, const T *LU, int lda, const v
   return cudaSuccess;
 }
 
+template <typename T>
+cudaError_t getrf_solve(cudaStream_t s, int n, T *A, int lda, void *scratch, int nrhs, T *B, int ldb, T *X, int ldx,
+                        bool keep_l, int *info_dev) {
+  if (n < 1) return cudaSuccess;
+  cudaError_t e = cudaMemsetAsync(info_dev + 1, 0, sizeof(int), s);
+  if (e != cudaSuccess) return e;
+  if ((e = factor<T>(s, n, A, lda, carve_lu(scratch, n), info_dev, keep_l, nrhs, B, ldb, X, ldx)) != cudaSuccess)
+    return e;
+  return triangular_solves<T>(s, n, nrhs, A, lda, X, ldx, false, true);
+}
+
+template <typename T>
+cudaError_t getrs(cudaStream_t s, int n, int nrhs, const T *LU, int lda, const void *scratch,
+                  const T *B, int ldb, T *X, int ldx, int *info_dev) {
+  if (n < 1 || nrhs < 1) return cudaSuccess;
+  const LuScratch sc = carve_lu(const_cast<void *>(scratch), n);
+  cudaError_t e = cudaMemsetAsync(info_dev, 0, sizeof(int), s);
+  if (e != cudaSuccess) return e;
+  {
+    const int gy = nrhs < 65535 ? nrhs : 65535;
+    gather_rows_kernel<T><<<dim3((n + 255) / 256, gy), 256, 0, s>>>(n, nrhs, sc.perm, B, ldb, X, ldx);
+    if ((e = launched()) != cudaSuccess) return e;
+  }
+  return triangular_solves<T>(s, n, nrhs, LU, lda, X, ldx, true, true);
+}
+
 #define CLM_INST_LU(T)                                                                            \
   template cudaError_t getrf<T>(cudaStream_t, int, T *, int, void *, int *);                     \
   template cudaError_t getrs<T>(cudaStream_t, int, int, const T *, int, const void *, const T *, \
-                                int, T *, int, int *);
+                                int, T *, int, int *);                                           \
+  template cudaError_t getrf_solve<T>(cudaStream_t, int, T *, int, void *, int, T *, int, T *, int, bool, int *);
 CLM_INST_LU(float)
 CLM_INST_LU(double)
 CLM_INST_LU(float2)

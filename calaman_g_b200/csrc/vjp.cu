@@ -199,8 +199,7 @@ calamanStatus_t vjp_api(calamanHandle_t blas, calamanStream_t stream, int n, con
     CLM_CUDA(launch_pade_split<T>(st, n, ws.T2, ws.LV, ws.T2, n, ws.LV));
     // R = q^-1 p; dR = q^-1 (dp - dq R)
     T *Rm = P[0], *Lm = M[0];
-    CLM_CUDA(getrf<T>(st, n, ws.V, n, ws.lu, d_info));
-    CLM_CUDA(getrs<T>(st, n, n, ws.V, n, ws.lu, ws.T1, n, Rm, n, d_info + 1));
+    CLM_CUDA(getrf_solve<T>(st, n, ws.V, n, ws.lu, n, ws.T1, n, Rm, n, true, d_info));
     CLM_CUDA(gemm_nn<T>(st, n, n, n, -1.0, ws.LV, n, Rm, n, 1.0, ws.T2, n));
     CLM_CUDA(getrs<T>(st, n, n, ws.V, n, ws.lu, ws.T2, n, Lm, n, d_info + 1));
 
