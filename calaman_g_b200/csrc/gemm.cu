@@ -449,6 +449,133 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// FP32 products on the FMA pipes (the polynomials without a lent workspace, the
+// public gemm): 64 x 64 tiles, 8 x 8 outputs a thread, so a k step is four
+// 16-byte shared loads for 64 FMAs (the form above, 4 x 4 with scalar loads, has
+// eight loads for 16 FMAs and is bound by them; 8 x 4 was still). Not larger
+// tiles, because the products of n = 1000 are 256 of these, 1.7 to an SM; to
+// have warps enough for the latencies all the same, a CTA is four groups of 64
+// threads that take a quarter of every k chunk each and add their sums at the
+// end. V16: A's and B's columns start 16-byte aligned.
+// 1000^3: 112 us (4 x 4), 81 us (8 x 4, one group), 70 us (8 x 4, two groups),
+// 66 us (this).
+template <bool V16>
+__global__ void __launch_bounds__(256)
+    sgemm_nn_kernel(int M, int N, int K, float alpha, const float *__restrict__ A, int lda,
+                    const float *__restrict__ B, int ldb, float beta, float *__restrict__ C, int ldc) {
+  constexpr int BM = 64, BN = 64, BK = 32;
+  __shared__ __align__(16) float sA[2][BK][BM];
+  __shared__ __align__(16) float sB[2][BK][BN + 4];
+  const int tid = threadIdx.x, group = tid >> 6;
+  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+  const int tx = tid & 7, ty = (tid >> 3) & 7;    // rows 4 tx + {0..3, 32..35}, columns 4 ty + the same
+  const int am = (tid & 15) * 4, ak = tid >> 4;   // A: 4 rows of depths ak, ak + 16
+  const int bk = (tid & 7) * 4, bn = tid >> 3;    // B: 4 depths of columns bn, bn + 32
+  float ra[2][4], rb[2][4];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int k = k0 + ak + 16 * q, m = m0 + am;
+      const float *pa = A + (std::size_t)k * lda + m;
+      if (V16 && k < K && m + 4 <= M) {
+        const float4 v = *reinterpret_cast<const float4 *>(pa);
+        ra[q][0] = v.x, ra[q][1] = v.y, ra[q][2] = v.z, ra[q][3] = v.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ra[q][e] = (k < K && m + e < M) ? pa[e] : 0.f;
+      }
+      const int n = n0 + bn + 32 * q, kk = k0 + bk;
+      const float *pb = B + (std::size_t)n * ldb + kk;
+      if (V16 && n < N && kk + 4 <= K) {
+        const float4 v = *reinterpret_cast<const float4 *>(pb);
+        rb[q][0] = v.x, rb[q][1] = v.y, rb[q][2] = v.z, rb[q][3] = v.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) rb[q][e] = (n < N && kk + e < K) ? pb[e] : 0.f;
+      }
+    }
+  };
+  auto stash = [&](int buf) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      *reinterpret_cast<float4 *>(&sA[buf][ak + 16 * q][am]) = make_float4(ra[q][0], ra[q][1], ra[q][2], ra[q][3]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) sB[buf][bk + e][bn + 32 * q] = rb[q][e];
+    }
+  };
+  float acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  const int KT = (K + BK - 1) / BK;
+  fetch(0);
+  stash(0);
+  __syncthreads();
+  for (int kt = 0; kt < KT; ++kt) {
+    const int cur = kt & 1;
+    if (kt + 1 < KT) fetch((kt + 1) * BK);
+#pragma unroll
+    for (int q = 0; q < BK / 4; ++q) {
+      const int kk = group * (BK / 4) + q;
+      const float4 a0 = *reinterpret_cast<const float4 *>(&sA[cur][kk][4 * tx]);
+      const float4 a1 = *reinterpret_cast<const float4 *>(&sA[cur][kk][32 + 4 * tx]);
+      const float4 b0 = *reinterpret_cast<const float4 *>(&sB[cur][kk][4 * ty]);
+      const float4 b1 = *reinterpret_cast<const float4 *>(&sB[cur][kk][32 + 4 * ty]);
+      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+      const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    }
+    if (kt + 1 < KT) stash(cur ^ 1);
+    __syncthreads();
+  }
+  // the groups' sums through shared memory, in group order (16 KB at a time)
+  float *const part = &sA[0][0][0] + (tid & 63);
+#pragma unroll 1
+  for (int g = 1; g < 4; ++g) {
+    if (group == g) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) part[(8 * i + j) * 64] = acc[i][j];
+    }
+    __syncthreads();
+    if (group == 0) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] += part[(8 * i + j) * 64];
+    }
+    __syncthreads();
+  }
+  if (group != 0) return;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    float old[4][8];  // 32 old C values in flight before their first store
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int m = m0 + 4 * tx + (i & 3) + 32 * (i >> 2), n = n0 + 4 * ty + j + 32 * h;
+        old[j][i] = (beta != 0.f && m < M && n < N) ? C[(std::size_t)n * ldc + m] : 0.f;
+      }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int m = m0 + 4 * tx + (i & 3) + 32 * (i >> 2), n = n0 + 4 * ty + j + 32 * h;
+        if (m < M && n < N) {
+          float v = acc[i][j + 4 * h] * alpha;
+          if (beta != 0.f) v = v + old[j][i] * beta;
+          C[(std::size_t)n * ldc + m] = v;
+        }
+      }
+  }
+}
+
 template <int BM, int BN, int WM, int WN, int STAGES, bool V16>
 cudaError_t run_dgemm(cudaStream_t s, int M, int N, int K, double alpha, const double *A, int lda,
                       const double *B, int ldb, double beta, double *C, int ldc, int splits = 1,
@@ -590,7 +717,9 @@ cudaError_t gemm_nn<float>(cudaStream_t s, int M, int N, int K, double alpha, co
   }
   return timed_launch(s, real_flops(M, N, K), [&] {
     dim3 grid((M + 63) / 64, (N + 63) / 64);
-    simt_gemm_nn_kernel<float><<<grid, 256, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+    const bool v16 = aligned16(A) && aligned16(B) && (lda % 4 == 0) && (ldb % 4 == 0);
+    auto kern = v16 ? sgemm_nn_kernel<true> : sgemm_nn_kernel<false>;
+    kern<<<grid, 256, 0, s>>>(M, N, K, (float)alpha, A, lda, B, ldb, (float)beta, C, ldc);
     return cudaGetLastError();
   });
 }
