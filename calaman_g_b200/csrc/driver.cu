@@ -170,6 +170,14 @@ calamanStatus_t expm_api(calamanHandle_t blas, calamanStream_t stream, int n, co
   const calamanExpmPlan_t chosen = plan_for<R>((R)norm);
   if (plan_out) *plan_out = chosen;
 
+  // Small matrices: everything after the norm in one kernel, faster than the
+  // general path's launches even as a graph (see small.cu). Not while GEMM
+  // launches are being timed, since it has none.
+  if (n <= expm_small_max_n<T>() && tl_timer == nullptr) {
+    CLM_CUDA(expm_small<T>(st, n, A, lda, E, lde, chosen.m, chosen.s, d_info));
+    return ok_status();
+  }
+
   // everything after the plan: launches only, no host synchronisation
   auto post = [&]() -> calamanStatus_t {
     const T *src = A;

@@ -127,6 +127,12 @@ template <typename T>
 cudaError_t getrf_solve(cudaStream_t s, int n, T *A, int lda, void *scratch, int nrhs, T *B, int ldb, T *X, int ldx,
                         bool keep_l, int *info_dev);
 
+// exp(A) of a matrix of at most expm_small_max_n in one kernel on one CTA:
+// E = r_m(2^-s A)^(2^s). info[0] as getrf's, info[1] = 0. E may alias A.
+template <typename T> int expm_small_max_n();
+template <typename T>
+cudaError_t expm_small(cudaStream_t st, int n, const T *A, int lda, T *E, int lde, int m, int s, int *info);
+
 // B = f op(A) for an rows x cols matrix A: op is the transpose, conjugated
 // when `conj` (complex types); B is cols x rows. A and B may not alias.
 template <typename T>

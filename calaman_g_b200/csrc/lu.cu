@@ -97,16 +97,6 @@ __host__ __device__ inline PanelSmem panel_smem(int rpc, int kb) {
   return o;
 }
 
-template <typename T> __device__ __forceinline__ T shfl(T v, int src);
-template <> __device__ __forceinline__ float shfl<float>(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-template <> __device__ __forceinline__ double shfl<double>(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-template <> __device__ __forceinline__ float2 shfl<float2>(float2 v, int src) {
-  return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
-}
-template <> __device__ __forceinline__ double2 shfl<double2>(double2 v, int src) {
-  return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
-}
-
 // (value, index) max with the first index winning ties
 __device__ __forceinline__ void argmax_merge(double &v, int &i, double ov, int oi) {
   if (ov > v || (ov == v && oi < i)) {

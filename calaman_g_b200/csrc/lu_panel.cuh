@@ -18,6 +18,16 @@ template <> __device__ __forceinline__ double safe_min<double>() { return DBL_MI
 template <> __device__ __forceinline__ double safe_min<float2>() { return FLT_MIN; }
 template <> __device__ __forceinline__ double safe_min<double2>() { return DBL_MIN; }
 
+template <typename T> __device__ __forceinline__ T shfl(T v, int src);
+template <> __device__ __forceinline__ float shfl<float>(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+template <> __device__ __forceinline__ double shfl<double>(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+template <> __device__ __forceinline__ float2 shfl<float2>(float2 v, int src) {
+  return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+template <> __device__ __forceinline__ double2 shfl<double2>(double2 v, int src) {
+  return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+
 // A pivot candidate: the IEEE-754 bits of |Re| + |Im| plus one (bits order
 // non-negative values as the values themselves), 0 for NaN, and the row's
 // current position. Float rows need 32 bits of key, the others 64. A thread

@@ -1,0 +1,79 @@
+"""expm of small matrices (one kernel on one CTA up to n = 64, complex 48)
+against the oracle, at the edges of its tile classes and of its range, every
+Pade degree, with squarings, padded leading dimensions and in place."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from helpers import NP_DTYPE, Runner, _dev, colmajor_buffer, from_buffer, rel_frob, scaled_random, vp
+
+pytestmark = pytest.mark.gpu
+
+# FP64 tiers: the library's bar. Single tiers: eps (6e-8) x the entries' growth in
+# the scaled evaluation (a few tens) x 2^s for the squarings of the quotient's error.
+BAR = {"d": 1e-12, "z": 1e-12, "s": 2e-5, "c": 2e-5}
+
+
+@pytest.fixture(scope="module")
+def run(cuda):
+    r = Runner()
+    yield r
+    r.close()
+
+
+@pytest.mark.parametrize("suf", ["s", "d", "c", "z"])
+@pytest.mark.parametrize("n", [1, 2, 3, 15, 16, 17, 32, 33, 47, 48, 49, 63, 64, 65])
+@pytest.mark.parametrize("norm", [0.01, 0.2, 0.9, 2.0, 3.5, 5.3, 40.0])  # m = 3 .. 13, s = 0 and s > 0
+def test_small_expm_matches_oracle(run, oracle, suf, n, norm):
+    a = scaled_random(n, norm, 77 * n + int(10 * norm), suf in "cz")
+    if norm > 6:
+        # Forming q = V - U loses a factor |V| / |q|, up to exp(|X|) with |X| up to 11 in the single tiers
+        # (2e4 eps for the scalar 10), for a positive real spectrum. On skew-Hermitian input |q| stays near
+        # |V|, so the bar holds: an imaginary spectrum for the large norm.
+        a = a - a.conj().T
+        a = a * (norm / max(np.abs(a).sum(axis=0).max(), 1e-300))
+    a = a.astype(NP_DTYPE[suf])
+    st, plan, e, _, info = run.expm(a, suf)
+    ref, oplan, _ = oracle.expm(a, single=suf in "sc")
+    assert st.ok and list(info) == [0, 0]
+    assert (plan.m, plan.s) == (oplan.m, oplan.s)
+    assert rel_frob(e, ref) <= BAR[suf]
+
+
+@pytest.mark.parametrize("suf", ["d", "z"])
+@pytest.mark.parametrize("n", [2, 10, 34, 48])
+def test_small_expm_pivots(run, oracle, suf, n):
+    """exp of rotations by almost pi: q_13 is close to exp(-A/2), a quarter turn with a diagonal near zero,
+    so every second column pivots."""
+    a = np.kron(np.eye(n // 2), np.array([[0.0, 3.1], [-3.1, 0.0]])).astype(NP_DTYPE[suf])
+    st, plan, e, _, info = run.expm(a, suf)
+    ref, _, _ = oracle.expm(a)
+    assert st.ok and list(info) == [0, 0] and plan.m == 13
+    assert rel_frob(e, ref) <= BAR[suf]
+
+
+@pytest.mark.parametrize("suf", ["s", "d", "c", "z"])
+@pytest.mark.parametrize("norm", [1.0, 30.0])
+def test_small_expm_in_place(run, oracle, suf, norm):
+    import torch
+
+    n, ld = 37, 41
+    a = scaled_random(n, norm, 5, suf in "cz")
+    a = (a - a.conj().T).astype(NP_DTYPE[suf])  # skew, as above
+    dA = _dev(colmajor_buffer(a, ld, suf))
+    before = dA.cpu().numpy().reshape(n, ld)[:, n:].copy()
+    b = ctypes.c_size_t()
+    assert getattr(run.lib, f"calaman_expm_bufferSize_{suf}")(run.h, n, ctypes.byref(b)).ok
+    w = run.workspace(b.value)
+    info = torch.full((2,), -9, dtype=torch.int32, device="cuda")
+    plan = run.capi.ExpmPlan()
+    st = getattr(run.lib, f"calaman_expm_{suf}")(
+        run.h, run.h, ctypes.c_void_p(run.stream), n, vp(dA), ld, vp(dA), ld, vp(w), b.value,
+        ctypes.cast(info.data_ptr(), run.capi.c_int_p), ctypes.byref(plan))
+    torch.cuda.synchronize()
+    assert st.ok and info.tolist() == [0, 0]
+    full = dA.cpu().numpy()
+    assert np.array_equal(full.reshape(n, ld)[:, n:], before)  # the padding rows are untouched
+    ref, _, _ = oracle.expm(a, single=suf in "sc")
+    assert rel_frob(from_buffer(full, n, ld), ref) <= BAR[suf]
