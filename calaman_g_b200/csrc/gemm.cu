@@ -532,22 +532,23 @@ __global__ void __launch_bounds__(256)
     if (kt + 1 < KT) stash(cur ^ 1);
     __syncthreads();
   }
-  // the groups' sums through shared memory, in group order (16 KB at a time)
-  float *const part = &sA[0][0][0] + (tid & 63);
+  // the groups' sums through shared memory: 2 and 3 onto 0 and 1, then 1 onto 0
+  float *const part = ((group & 1) ? &sB[0][0][0] : &sA[0][0][0]) + (tid & 63);
 #pragma unroll 1
-  for (int g = 1; g < 4; ++g) {
-    if (group == g) {
+  for (int g = 2; g > 0; g >>= 1) {
+    float *const at = g == 2 ? part : &sA[0][0][0] + (tid & 63);
+    if (group >= g && group < 2 * g) {
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) part[(8 * i + j) * 64] = acc[i][j];
+        for (int j = 0; j < 8; ++j) at[(8 * i + j) * 64] = acc[i][j];
     }
     __syncthreads();
-    if (group == 0) {
+    if (group < g) {
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] += part[(8 * i + j) * 64];
+        for (int j = 0; j < 8; ++j) acc[i][j] += at[(8 * i + j) * 64];
     }
     __syncthreads();
   }
