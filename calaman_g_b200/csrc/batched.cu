@@ -978,13 +978,18 @@ struct ExpmLu {
 
 // kFactor: LU with partial pivoting of Q, then the solve; otherwise the solve
 // alone with factors and permutation from an earlier kFactor launch.
-template <typename Item, typename T, typename Lu, bool kFactor, int NT>
+// kOverlap: see launch_lu (a template argument, since the extra instructions
+// alone made the FP32 kernel of a large batch 5 % slower).
+template <typename Item, typename T, typename Lu, bool kFactor, int NT, bool kOverlap>
 __global__ void __launch_bounds__(NT, BLuOcc<T, NT, Lu>::kMinBlocks)
     g_lu_kernel(const Item *__restrict__ items, const BPlan *__restrict__ plans, int *__restrict__ info,
                 int mode) {
   using R = typename elem<T>::real;
-  const Item it = items[blockIdx.x];
-  const BPlan pl = plans[blockIdx.x];
+  // the next size class may start beside this one
+  if constexpr (kOverlap) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int item = kOverlap ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+  const Item it = items[item];
+  const BPlan pl = plans[item];
   const int n = it.n;
   const LuOps<T> lo = Lu::ops(it, pl, mode);
   T *Q = lo.Q;
@@ -1229,6 +1234,8 @@ __global__ void __launch_bounds__(NT, BLuOcc<T, NT, Lu>::kMinBlocks)
     blk_rows<false, T, NT>(D, ldd, k, jb, n, n, 0, blk);
     cta_update<T, NT>(D, ldd, 0, k, 0, n, Q + (std::size_t)k * n, n, jb, blk, Ls);
   }
+  // this launch is over only when the size class before it is
+  if constexpr (kOverlap) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 template <typename T, int NT> constexpr std::size_t lu_smem_bytes() {
@@ -1239,20 +1246,28 @@ template <typename T, int NT> constexpr std::size_t lu_smem_bytes() {
 // matrices that share a CTA size: by default 64-thread CTAs for n <= 64, 128
 // for n <= 128, 256 above (small matrices pack more CTAs per SM); a schedule
 // (lu_threads[ceil(n / 16)], each >= n) may choose per size bucket.
+// A batch of few matrices (up to kOverlapItems, some two to eight CTAs per SM)
+// leaves SMs idle at the end of every launch, and the launches are of unlike
+// length: there the classes run in descending size, the longest CTAs first, each
+// launch beside the one before it (programmatic dependent launch; a launch ends
+// only after the one before, so the phases behind wait for all of them). 500
+// float64 matrices, n = 3 .. 200: 2622 -> 2226 us. Thousands of matrices fill
+// every launch nearly to its end; they keep the plain launches.
+constexpr int kOverlapItems = 8 * 148;
 template <typename Item, typename T, typename Lu, bool kFactor>
 cudaError_t launch_lu(cudaStream_t st, const Item *items, const BPlan *plans, int *info, int mode,
                       const std::vector<int> &ns, const int *lu_threads = nullptr) {
   const int count = (int)ns.size();
+  const bool overlap = count <= kOverlapItems;
   auto threads_of = [&](int n) {
     const int d = n <= 64 ? 64 : n <= 128 ? 128 : 256;
     if (lu_threads == nullptr) return d;
     const int t = lu_threads[(n + 15) / 16];
     return (t == 64 || t == 128 || t == 256) && t >= n ? t : d;
   };
-  auto one = [&](auto nt_tag, int from, int to) -> cudaError_t {
+  auto one = [&](auto nt_tag, auto overlap_tag, int from, int to) -> cudaError_t {
     constexpr int NT = decltype(nt_tag)::value;
-    if (to <= from) return cudaSuccess;
-    auto kern = g_lu_kernel<Item, T, Lu, kFactor, NT>;
+    auto kern = g_lu_kernel<Item, T, Lu, kFactor, NT, decltype(overlap_tag)::value>;
     constexpr std::size_t smem = lu_smem_bytes<T, NT>();
     static bool configured = false;  // once, before any graph capture of a call
     if (!configured) {
@@ -1263,20 +1278,41 @@ cudaError_t launch_lu(cudaStream_t st, const Item *items, const BPlan *plans, in
       if (e != cudaSuccess) return e;
       configured = true;
     }
-    kern<<<to - from, NT, smem, st>>>(items + from, plans + from, info, mode);
-    return launched();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(to - from, 1, 1);
+    cfg.blockDim = dim3(NT, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap && to < count ? 1 : 0;  // the first launch waits for the phases before
+    note_launch();
+    return cudaLaunchKernelEx(&cfg, kern, items + from, plans + from, info, mode);
   };
-  for (int from = 0; from < count;) {
-    const int nt = threads_of(ns[from]);
-    int to = from + 1;
-    while (to < count && threads_of(ns[to]) == nt) ++to;
-    cudaError_t e = nt == 64    ? one(std::integral_constant<int, 64>{}, from, to)
-                    : nt == 128 ? one(std::integral_constant<int, 128>{}, from, to)
-                                : one(std::integral_constant<int, 256>{}, from, to);
-    if (e != cudaSuccess) return e;
-    from = to;
+  auto run = [&](int from, int to) -> cudaError_t {
+    auto by_size = [&](auto tag) -> cudaError_t {
+      const int nt = threads_of(ns[from]);
+      return nt == 64    ? one(std::integral_constant<int, 64>{}, tag, from, to)
+             : nt == 128 ? one(std::integral_constant<int, 128>{}, tag, from, to)
+                         : one(std::integral_constant<int, 256>{}, tag, from, to);
+    };
+    return overlap ? by_size(std::true_type{}) : by_size(std::false_type{});
+  };
+  cudaError_t e = cudaSuccess;
+  if (overlap) {
+    for (int to = count, from; to > 0 && e == cudaSuccess; to = from) {
+      for (from = to - 1; from > 0 && threads_of(ns[from - 1]) == threads_of(ns[to - 1]);) --from;
+      e = run(from, to);
+    }
+  } else {
+    for (int from = 0, to; from < count && e == cudaSuccess; from = to) {
+      for (to = from + 1; to < count && threads_of(ns[to]) == threads_of(ns[from]);) ++to;
+      e = run(from, to);
+    }
   }
-  return cudaSuccess;
+  return e;
 }
 
 // ---- precision conversion between the caller's buffers and FP64 copies ----
