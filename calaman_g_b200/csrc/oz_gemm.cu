@@ -283,72 +283,89 @@ __global__ void __launch_bounds__(kOzThreads, 1)
   }
 }
 
-// ---- operand maxima -----------------------------------------------------------
-// Largest |A[r,k]| over k for every row r of the caller's A (complex: the
-// larger of |Re| and |Im|), as the bits of a non-negative double. Block:
-// 32 rows x 32 k-lanes, the k-lanes reduced through shared memory.
+// Largest magnitude (complex: of |Re| and |Im|) of every row of A, then of every
+// column of B, as bits; with diag the diagonals are left out. Blocks [0, rblocks)
+// take eight rows each (64-byte pieces of a column, 64 columns in flight), the
+// others sixteen columns, a warp each. One launch of 2048 / 8 + 2048 / 16 blocks
+// at n = 2048, where 32 rows per block had left more than half of the SMs idle:
+// 41 us (two launches) -> 19 us.
+constexpr int kMaxThreads = 512;
 template <typename T>
-__global__ void __launch_bounds__(1024) oz_row_max_kernel(int M, int K, const T *__restrict__ A, int lda,
-                                                          int diag, unsigned long long *__restrict__ amax) {
-  __shared__ double red[32][33];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int r = blockIdx.x * 32 + tx;
+__global__ void __launch_bounds__(kMaxThreads)
+    oz_max_kernel(int M, int N, int K, const T *__restrict__ A, int lda, const T *__restrict__ B, int ldb, int diag,
+                  int rblocks, unsigned long long *__restrict__ amax, unsigned long long *__restrict__ bmax) {
+  auto magnitude = [](T x) -> double {
+    if constexpr (elem<T>::complex) return fmax(fabs((double)x.x), fabs((double)x.y));
+    else return fabs((double)x);
+  };
   double m = 0.0;
-  if (r < M)
-    for (int k = ty; k < K; k += 32) {
-      const T x = A[(std::size_t)k * lda + r];
-      double v;
-      if constexpr (elem<T>::complex) v = fmax(fabs((double)x.x), fabs((double)x.y));
-      else v = fabs((double)x);
-      m = fmax(m, (diag && k == r) ? 0.0 : v);
+  if ((int)blockIdx.x < rblocks) {
+    __shared__ double red[kMaxThreads / 32][8];
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
+    const int r = blockIdx.x * 8 + tx;
+    if (r < M) {
+#pragma unroll 8
+      for (int k = ty; k < K; k += kMaxThreads / 8) {
+        const double v = magnitude(A[(std::size_t)k * lda + r]);
+        m = fmax(m, (diag && k == r) ? 0.0 : v);
+      }
     }
-  red[ty][tx] = m;
-  __syncthreads();
-  if (ty == 0 && r < M) {
-    for (int j = 1; j < 32; ++j) m = fmax(m, red[j][tx]);
-    const unsigned long long bits = (unsigned long long)__double_as_longlong(m);
-    amax[r] = bits;
-    if constexpr (elem<T>::complex) amax[M + r] = bits;
-  }
-}
-
-// Largest |B[k,c]| over k for every column c (complex: |Re| and |Im|): one
-// warp per column.
-template <typename T>
-__global__ void __launch_bounds__(256) oz_col_max_kernel(int K, int N, const T *__restrict__ B, int ldb,
-                                                         int diag, unsigned long long *__restrict__ bmax) {
-  const int c = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (c >= N) return;
-  double m = 0.0;
-  for (int k = lane; k < K; k += 32) {
-    const T x = B[(std::size_t)c * ldb + k];
-    double v;
-    if constexpr (elem<T>::complex) v = fmax(fabs((double)x.x), fabs((double)x.y));
-    else v = fabs((double)x);
-    m = fmax(m, (diag && k == c) ? 0.0 : v);
-  }
+    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, 8));
+    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, 16));
+    if ((threadIdx.x & 31) < 8) red[threadIdx.x >> 5][tx] = m;
+    __syncthreads();
+    if (threadIdx.x < 8 && r < M) {
+      for (int j = 0; j < kMaxThreads / 32; ++j) m = fmax(m, red[j][tx]);
+      const unsigned long long bits = (unsigned long long)__double_as_longlong(m);
+      amax[r] = bits;
+      if constexpr (elem<T>::complex) amax[M + r] = bits;
+    }
+  } else {
+    const int c = (blockIdx.x - rblocks) * (kMaxThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (c >= N) return;
+#pragma unroll 8
+    for (int k = lane; k < K; k += 32) {
+      const double v = magnitude(B[(std::size_t)c * ldb + k]);
+      m = fmax(m, (diag && k == c) ? 0.0 : v);
+    }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (lane == 0) bmax[c] = (unsigned long long)__double_as_longlong(m);
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) bmax[c] = (unsigned long long)__double_as_longlong(m);
+  }
 }
 
-// The ks digits of 16 consecutive values x[0..15] scaled by 2^(7 - e),
-// packed little-endian into 16 bytes per digit plane.
+// The ks digits of 16 consecutive values x[0..15], |x| < 2^e, packed
+// little-endian into 16 bytes per digit plane. The digits of a value are the
+// 7-bit fields of floor(|x| 2^(7 ks - e)), an integer of 7 ks <= 56 bits, with
+// the value's sign: one FP64 conversion per value (a truncation per digit in
+// FP64 had been the kernels' bound; with the coalesced reads of B, at n = 2048:
+// A 32 -> 26 us, B 28 -> 14 us). The power of two is applied in two factors,
+// since 7 ks - e may exceed the exponent range; both steps are exact except
+// below one, where the floor is zero anyway.
 template <int KS>
 __device__ __forceinline__ void digits16(const double (&x)[16], int e, uint4 (&out)[KS]) {
+  const int sh = 7 * KS - e, s1 = sh / 2, s2 = sh - s1;
+  const double f1 = __longlong_as_double((long long)(1023 + s1) << 52);
+  const double f2 = __longlong_as_double((long long)(1023 + s2) << 52);
   uint32_t w[KS][4];
 #pragma unroll
-  for (int i = 0; i < KS; ++i)
+  for (int q = 0; q < 4; ++q) {
+    unsigned long long v[4];
+    uint32_t neg = 0u;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) w[i][q] = 0u;
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    double y = ldexp(x[j], 7 - e);  // |y| < 128
+    for (int j = 0; j < 4; ++j) {
+      const double y = x[4 * q + j];
+      v[j] = (unsigned long long)__double2ull_rz(fabs(y) * f1 * f2);
+      if (y < 0.0) neg |= 0xffu << (8 * j);
+    }
 #pragma unroll
     for (int i = 0; i < KS; ++i) {
-      const double d = trunc(y);
-      w[i][j >> 2] |= ((uint32_t)(int)d & 0xffu) << (8 * (j & 3));
-      y = (y - d) * 128.0;
+      uint32_t p = 0u;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) p |= ((uint32_t)(v[j] >> (7 * (KS - 1 - i))) & 127u) << (8 * j);
+      // bytes under `neg` negated: complement, plus one without carries between bytes
+      const uint32_t t = p ^ neg;
+      w[i][q] = ((t & 0x7f7f7f7fu) + (neg & 0x01010101u)) ^ (t & 0x80808080u);
     }
   }
 #pragma unroll
@@ -402,19 +419,18 @@ __global__ void __launch_bounds__(256) oz_slice_a_kernel(int M, int K, const T *
 }
 
 // B digits: planes [ks][Np][Kp], row c = column c of the real B operand (for
-// complex, [Br; Bi]); each thread cuts 16 consecutive k of one column.
+// complex, [Br; Bi]). Block: 16 columns x 256 k through a shared tile (coalesced
+// reads along k), each thread then cuts 16 consecutive k of one column.
 template <typename T, int KS>
-__global__ void __launch_bounds__(128) oz_slice_b_kernel(int K, int N, const T *__restrict__ B, int ldb,
+__global__ void __launch_bounds__(256) oz_slice_b_kernel(int K, int N, const T *__restrict__ B, int ldb,
                                                          int Kr, int Np, int Kp, int diag,
                                                          const unsigned long long *__restrict__ bmax,
                                                          int8_t *__restrict__ digits) {
-  const int c = blockIdx.y;
-  const int k0 = (blockIdx.x * 128 + threadIdx.x) * 16;
-  if (k0 >= Kp) return;
-  double x[16];
+  __shared__ double tile[16][16 * 17];  // groups of 16 k, 17 apart
+  const int t = threadIdx.x, c0 = blockIdx.y * 16, k0 = blockIdx.x * 256;
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const int k = k0 + j;
+  for (int cc = 0; cc < 16; ++cc) {
+    const int c = c0 + cc, k = k0 + t;
     double v = 0.0;
     if (c < N && k < Kr && !(diag && (k < K ? k : k - K) == c)) {
       if constexpr (elem<T>::complex) {
@@ -424,13 +440,19 @@ __global__ void __launch_bounds__(128) oz_slice_b_kernel(int K, int N, const T *
         v = (double)B[(std::size_t)c * ldb + k];
       }
     }
-    x[j] = v;
+    tile[cc][(t >> 4) * 17 + (t & 15)] = v;
   }
+  __syncthreads();
+  const int kg = t & 15, cc = t >> 4, c = c0 + cc;
+  if (k0 + kg * 16 >= Kp) return;
+  double x[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) x[j] = tile[cc][kg * 17 + j];
   const int e = c < N ? exp_of_bits(bmax[c]) : 0;
   uint4 d[KS];
   digits16<KS>(x, e, d);
   const std::size_t plane = (std::size_t)Np * Kp;
-  int8_t *dst = digits + (std::size_t)c * Kp + k0;
+  int8_t *dst = digits + (std::size_t)c * Kp + k0 + kg * 16;
 #pragma unroll
   for (int i = 0; i < KS; ++i) *reinterpret_cast<uint4 *>(dst + i * plane) = d[i];
 }
@@ -483,14 +505,13 @@ cudaError_t slice_operands(cudaStream_t s, int M, int N, int K, const T *A, int 
   auto *da = reinterpret_cast<int8_t *>(w + L.a_off);
   auto *db = reinterpret_cast<int8_t *>(w + L.b_off);
   cudaError_t e;
-  oz_row_max_kernel<T><<<(M + 31) / 32, 1024, 0, s>>>(M, K, A, lda, diag, amax);
-  if ((e = launched()) != cudaSuccess) return e;
-  oz_col_max_kernel<T><<<(N + 7) / 8, 256, 0, s>>>(K, N, B, ldb, diag, bmax);
+  const int rblocks = (M + 7) / 8, cblocks = (N + kMaxThreads / 32 - 1) / (kMaxThreads / 32);
+  oz_max_kernel<T><<<rblocks + cblocks, kMaxThreads, 0, s>>>(M, N, K, A, lda, B, ldb, diag, rblocks, amax, bmax);
   if ((e = launched()) != cudaSuccess) return e;
   oz_slice_a_kernel<T, KS><<<dim3(L.Mrp / 64, L.Kp / 64), 256, 0, s>>>(M, K, A, lda, L.Mrows, L.Kr, L.Mrp,
                                                                        L.Kp, diag, amax, da);
   if ((e = launched()) != cudaSuccess) return e;
-  oz_slice_b_kernel<T, KS><<<dim3((L.Kp / 16 + 127) / 128, L.Np), 128, 0, s>>>(K, N, B, ldb, L.Kr, L.Np, L.Kp,
+  oz_slice_b_kernel<T, KS><<<dim3((L.Kp + 255) / 256, L.Np / 16), 256, 0, s>>>(K, N, B, ldb, L.Kr, L.Np, L.Kp,
                                                                                diag, bmax, db);
   return launched();
 }

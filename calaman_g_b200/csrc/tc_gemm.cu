@@ -29,6 +29,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -211,11 +212,21 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 // ---- operand split kernels --------------------------------------------------
-__device__ __forceinline__ void split3(float x, __nv_bfloat16 &h, __nv_bfloat16 &m, __nv_bfloat16 &l) {
-  h = __float2bfloat16_rn(x);
-  const float r = x - __bfloat162float(h);
-  m = __float2bfloat16_rn(r);
-  l = __float2bfloat16_rn(r - __bfloat162float(m));
+// Eight values split into bf16 parts, packed 16 bytes a part.
+__device__ __forceinline__ void split8(const float (&x)[8], uint4 (&part)[3]) {
+  uint32_t w[3][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
+    const float r0 = x[2 * i] - __low2float(h), r1 = x[2 * i + 1] - __high2float(h);
+    const __nv_bfloat162 m = __floats2bfloat162_rn(r0, r1);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(r0 - __low2float(m), r1 - __high2float(m));
+    w[0][i] = *reinterpret_cast<const uint32_t *>(&h);
+    w[1][i] = *reinterpret_cast<const uint32_t *>(&m);
+    w[2][i] = *reinterpret_cast<const uint32_t *>(&l);
+  }
+#pragma unroll
+  for (int p = 0; p < 3; ++p) part[p] = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
 }
 
 // Element (m, k) of the real A operand: A itself, or for complex (Mc > 0,
@@ -232,56 +243,68 @@ __device__ __forceinline__ float a_at(const T *A, int lda, int Mc, int Kc, int m
 }
 
 // A (M x K real rows; column-major, lda) -> parts[p][row][k], rows of Kpad,
-// Mpad rows per part; the transpose goes through a 32 x 33 shared tile.
+// Mpad rows per part (multiples of 64): 64 x 64 through a shared tile, each
+// thread then writes 16-byte pieces of 8 k (2-byte stores had held this kernel
+// at half of the memory rate: 4096 x 4096 54 us -> 25 us; split_b 58 -> 25 us).
 template <typename T>
-__global__ void split_a_kernel(int M, int K, const T *__restrict__ A, int lda, int Mc, int Kc, int Mpad,
-                               int Kpad, int nparts, __nv_bfloat16 *__restrict__ parts) {
-  __shared__ float tile[32][33];
-  const int mb = blockIdx.x * 32, kb = blockIdx.y * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8 threads
-  for (int r = ty; r < 32; r += 8) {  // read: consecutive m along tx
-    const int m = mb + tx, k = kb + r;
-    tile[r][tx] = (m < M && k < K) ? a_at<T>(A, lda, Mc, Kc, m, k) : 0.f;
+__global__ void __launch_bounds__(256)
+    split_a_kernel(int M, int K, const T *__restrict__ A, int lda, int Mc, int Kc, int Mpad, int Kpad, int nparts,
+                   __nv_bfloat16 *__restrict__ parts) {
+  __shared__ float tile[64][65];
+  const int mb = blockIdx.x * 64, kb = blockIdx.y * 64, t = threadIdx.x;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {  // read: consecutive m along the lanes
+    const int r = t & 63, kk = (t >> 6) + 4 * q, m = mb + r, k = kb + kk;
+    tile[kk][r] = (m < M && k < K) ? a_at<T>(A, lda, Mc, Kc, m, k) : 0.f;
   }
   __syncthreads();
   const std::size_t part_stride = (std::size_t)Mpad * Kpad;
-  for (int r = ty; r < 32; r += 8) {  // write: consecutive k along tx
-    const int m = mb + r, k = kb + tx;
-    if (m < Mpad && k < Kpad) {
-      __nv_bfloat16 h, mm, l;
-      split3(tile[tx][r], h, mm, l);
-      const std::size_t at = (std::size_t)m * Kpad + k;
-      parts[at] = h;
-      parts[part_stride + at] = mm;
-      if (nparts > 2) parts[2 * part_stride + at] = l;
-    }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {  // write: eight lanes to the 128 bytes of a row
+    const int kg = (t & 7) * 8, r = (t >> 3) + 32 * q;
+    float x[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = tile[kg + j][r];
+    uint4 v[3];
+    split8(x, v);
+    __nv_bfloat16 *at = parts + (std::size_t)(mb + r) * Kpad + kb + kg;
+    *reinterpret_cast<uint4 *>(at) = v[0];
+    *reinterpret_cast<uint4 *>(at + part_stride) = v[1];
+    if (nparts > 2) *reinterpret_cast<uint4 *>(at + 2 * part_stride) = v[2];
   }
 }
 
 // B (K x N real; column-major, ldb; for complex [Br; Bi] with Kc the complex
-// depth) -> parts[p][col][k]: already K-contiguous.
+// depth) -> parts[p][col][k]: already K-contiguous, 8 k a thread.
 template <typename T>
-__global__ void split_b_kernel(int K, int N, const T *__restrict__ B, int ldb, int Kc, int Npad,
-                               int Kpad, int nparts, __nv_bfloat16 *__restrict__ parts) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= Kpad) return;
+__global__ void __launch_bounds__(256)
+    split_b_kernel(int K, int N, const T *__restrict__ B, int ldb, int Kc, int Npad, int Kpad, int nparts,
+                   __nv_bfloat16 *__restrict__ parts) {
   const std::size_t part_stride = (std::size_t)Npad * Kpad;
-  for (int n = blockIdx.y; n < Npad; n += gridDim.y) {
-    float x = 0.f;
-    if (k < K && n < N) {
-      if constexpr (std::is_same<T, float2>::value) {
-        const float2 z = B[(std::size_t)n * ldb + (k < Kc ? k : k - Kc)];
-        x = k < Kc ? z.x : z.y;
-      } else {
-        x = B[(std::size_t)n * ldb + k];
+  const int pieces = Kpad >> 3;  // per column
+  const long long total = (long long)Npad * pieces;
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < total; i += gridDim.x * 256ll) {
+    const int n = (int)(i / pieces), k0 = (int)(i - (long long)n * pieces) * 8;
+    float x[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int k = k0 + j;
+      x[j] = 0.f;
+      if (k < K && n < N) {
+        if constexpr (std::is_same<T, float2>::value) {
+          const float2 z = B[(std::size_t)n * ldb + (k < Kc ? k : k - Kc)];
+          x[j] = k < Kc ? z.x : z.y;
+        } else {
+          x[j] = B[(std::size_t)n * ldb + k];
+        }
       }
     }
-    __nv_bfloat16 h, m, l;
-    split3(x, h, m, l);
-    const std::size_t at = (std::size_t)n * Kpad + k;
-    parts[at] = h;
-    parts[part_stride + at] = m;
-    if (nparts > 2) parts[2 * part_stride + at] = l;
+    uint4 v[3];
+    split8(x, v);
+    __nv_bfloat16 *at = parts + (std::size_t)n * Kpad + k0;
+    *reinterpret_cast<uint4 *>(at) = v[0];
+    *reinterpret_cast<uint4 *>(at + part_stride) = v[1];
+    if (nparts > 2) *reinterpret_cast<uint4 *>(at + 2 * part_stride) = v[2];
   }
 }
 
@@ -316,21 +339,12 @@ struct RankParams {
 
 // One 16-byte piece (8 consecutive k of one row) of every part tile.
 __device__ __forceinline__ void store_parts(unsigned char *tile, int nparts, int row, int piece, const float (&x)[8]) {
-  uint32_t h[4], m[4], l[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const __nv_bfloat162 hh = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
-    const float r0 = x[2 * i] - __low2float(hh), r1 = x[2 * i + 1] - __high2float(hh);
-    const __nv_bfloat162 mm = __floats2bfloat162_rn(r0, r1);
-    const __nv_bfloat162 ll = __floats2bfloat162_rn(r0 - __low2float(mm), r1 - __high2float(mm));
-    h[i] = *reinterpret_cast<const uint32_t *>(&hh);
-    m[i] = *reinterpret_cast<const uint32_t *>(&mm);
-    l[i] = *reinterpret_cast<const uint32_t *>(&ll);
-  }
+  uint4 v[3];
+  split8(x, v);
   unsigned char *at = tile + row * 128 + ((piece ^ (row & 7)) << 4);
-  *reinterpret_cast<uint4 *>(at) = make_uint4(h[0], h[1], h[2], h[3]);
-  *reinterpret_cast<uint4 *>(at + kPart) = make_uint4(m[0], m[1], m[2], m[3]);
-  if (nparts > 2) *reinterpret_cast<uint4 *>(at + 2 * kPart) = make_uint4(l[0], l[1], l[2], l[3]);
+  *reinterpret_cast<uint4 *>(at) = v[0];
+  *reinterpret_cast<uint4 *>(at + kPart) = v[1];
+  if (nparts > 2) *reinterpret_cast<uint4 *>(at + 2 * kPart) = v[2];
 }
 
 template <bool CPLX>
@@ -542,15 +556,13 @@ cudaError_t tc_gemm_run(cudaStream_t s, int Mc, int N, int Kc, double alpha, con
   auto *pb = reinterpret_cast<__nv_bfloat16 *>(w + 256 + L.a_bytes);
 
   cudaError_t e;
-  split_a_kernel<T><<<dim3(L.Mpad / 32, L.Kpad / 32), 256, 0, s>>>(M, K, A, lda, Mc, Kc, L.Mpad, L.Kpad, nparts,
+  split_a_kernel<T><<<dim3(L.Mpad / 64, L.Kpad / 64), 256, 0, s>>>(M, K, A, lda, Mc, Kc, L.Mpad, L.Kpad, nparts,
                                                                    pa);
   if ((e = launched()) != cudaSuccess) return e;
-  {
-    const int gy = L.Npad < 65535 ? L.Npad : 65535;
-    split_b_kernel<T><<<dim3((L.Kpad + 255) / 256, gy), 256, 0, s>>>(K, N, B, ldb, Kc, L.Npad, L.Kpad, nparts,
-                                                                     pb);
-    if ((e = launched()) != cudaSuccess) return e;
-  }
+  const long long pieces = (long long)L.Npad * (L.Kpad / 8);
+  split_b_kernel<T><<<(unsigned)std::min<long long>((pieces + 255) / 256, 1 << 20), 256, 0, s>>>(
+      K, N, B, ldb, Kc, L.Npad, L.Kpad, nparts, pb);
+  if ((e = launched()) != cudaSuccess) return e;
 
   CUtensorMap ma, mb;
   if (!make_map(&ma, pa, (long long)nparts * L.Mpad, L.Kpad, TM)) return cudaErrorNotSupported;
