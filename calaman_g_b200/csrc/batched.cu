@@ -124,6 +124,70 @@ __global__ void __launch_bounds__(256) b_scale_kernel(const BItem<T, Wd> *__rest
   }
 }
 
+// W consecutive elements, moved as one 16-byte piece where W fills it. The
+// elementwise phases below are bound by memory and by the loads in flight: where
+// a matrix's n^2 is a multiple of the piece (ld = n) and its buffers are aligned,
+// a thread takes a piece per step, else one element.
+template <typename T> constexpr int ew_piece() { return 16 / (int)sizeof(T); }
+template <int W, typename T>
+struct Pack {
+  T e[W];
+};
+template <int W, typename T>
+__device__ __forceinline__ Pack<W, T> ew_load(const T *p) {
+  Pack<W, T> v;
+  if constexpr (W > 1) {
+    union {
+      uint4 u;
+      T e[W];
+    } w;
+    w.u = *reinterpret_cast<const uint4 *>(p);
+#pragma unroll
+    for (int i = 0; i < W; ++i) v.e[i] = w.e[i];
+  } else {
+    v.e[0] = *p;
+  }
+  return v;
+}
+template <int W, typename T>
+__device__ __forceinline__ void ew_store(T *p, const Pack<W, T> &v) {
+  if constexpr (W > 1) {
+    union {
+      uint4 u;
+      T e[W];
+    } w;
+#pragma unroll
+    for (int i = 0; i < W; ++i) w.e[i] = v.e[i];
+    *reinterpret_cast<uint4 *>(p) = w.u;
+  } else {
+    *p = v.e[0];
+  }
+}
+// body(std::integral_constant<int, W>, e) for every piece of this CTA's chunk of
+// nn elements; buf: one of the matrix's buffers, which all lie 256 bytes apart
+template <typename T, typename F>
+__device__ __forceinline__ void ew_for(const T *buf, int nn, F &&body) {
+  constexpr int V = ew_piece<T>();
+  const int end = min(nn, (int)(blockIdx.y + 1) * kEwChunk);
+  if (nn % V == 0 && (reinterpret_cast<std::uintptr_t>(buf) & 15) == 0) {
+    for (int e = blockIdx.y * kEwChunk + threadIdx.x * V; e < end; e += blockDim.x * V)
+      body(std::integral_constant<int, V>{}, e);
+  } else {
+    for (int e = blockIdx.y * kEwChunk + threadIdx.x; e < end; e += blockDim.x)
+      body(std::integral_constant<int, 1>{}, e);
+  }
+}
+// body(i, diagonal) for the elements e .. e + W - 1 of an n x n matrix
+template <int W, typename F>
+__device__ __forceinline__ void ew_diag(int e, int n, F &&body) {
+  int c = e / n, r = e - c * n;
+#pragma unroll
+  for (int i = 0; i < W; ++i) {
+    body(i, r == c);
+    if (++r == n) r = 0, ++c;
+  }
+}
+
 // V, W from the even powers (m < 13); for m = 13 also the odd temp T and the
 // even temp (into P3, unused at m = 13):
 //   T = b9 A2 + b11 A4 + b13 A6,  W = b1 I + b3 A2 + b5 A4 + b7 A6,
@@ -135,59 +199,70 @@ __global__ void __launch_bounds__(256) b_even_odd_kernel(const BItem<T, Wd> *__r
   const BItem<T, Wd> it = items[blockIdx.x];
   const BPlan pl = plans[blockIdx.x];
   const double *b = c_pade[degree_slot(pl.m)];
-  const int n = it.n, nn = n * n;
-  const int end = min(nn, (int)(blockIdx.y + 1) * kEwChunk);
+  const int n = it.n;
   const T *P[4] = {it.P0, it.P1, it.P2, it.P3};
-  for (int e = blockIdx.y * kEwChunk + threadIdx.x; e < end; e += blockDim.x) {
-    const int c = e / n, r = e - c * n;
-    const bool diag = r == c;
+  ew_for<T>(it.V, n * n, [&](auto piece, int e) {
+    constexpr int W = decltype(piece)::value;
     if (pl.m != 13) {
-      T v = elem<T>::zero(), w = elem<T>::zero();
+      Pack<W, T> v, w;
+#pragma unroll
+      for (int i = 0; i < W; ++i) v.e[i] = w.e[i] = elem<T>::zero();
       for (int k = 0; k < pl.np; ++k) {
-        const T x = P[k][e];
-        v = rfma((R)b[2 * k + 2], x, v);
-        w = rfma((R)b[2 * k + 3], x, w);
+        const Pack<W, T> x = ew_load<W>(P[k] + e);
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          v.e[i] = rfma((R)b[2 * k + 2], x.e[i], v.e[i]);
+          w.e[i] = rfma((R)b[2 * k + 3], x.e[i], w.e[i]);
+        }
       }
-      if (diag) {
-        v = add_real(v, (R)b[0]);
-        w = add_real(w, (R)b[1]);
-      }
-      it.V[e] = v;
-      it.W[e] = w;
+      ew_diag<W>(e, n, [&](int i, bool diag) {
+        if (diag) {
+          v.e[i] = add_real(v.e[i], (R)b[0]);
+          w.e[i] = add_real(w.e[i], (R)b[1]);
+        }
+      });
+      ew_store<W>(it.V + e, v);
+      ew_store<W>(it.W + e, w);
     } else {
-      const T x1 = it.P0[e], x2 = it.P1[e], x3 = it.P2[e];
-      T t = scale(x1, (R)b[9]), w = scale(x1, (R)b[3]), z = scale(x1, (R)b[8]), v = scale(x1, (R)b[2]);
-      t = rfma((R)b[11], x2, t);
-      w = rfma((R)b[5], x2, w);
-      z = rfma((R)b[10], x2, z);
-      v = rfma((R)b[4], x2, v);
-      t = rfma((R)b[13], x3, t);
-      w = rfma((R)b[7], x3, w);
-      z = rfma((R)b[12], x3, z);
-      v = rfma((R)b[6], x3, v);
-      if (diag) {
-        w = add_real(w, (R)b[1]);
-        v = add_real(v, (R)b[0]);
+      const Pack<W, T> x1 = ew_load<W>(it.P0 + e), x2 = ew_load<W>(it.P1 + e), x3 = ew_load<W>(it.P2 + e);
+      Pack<W, T> t, w, z, v;
+#pragma unroll
+      for (int i = 0; i < W; ++i) {
+        t.e[i] = rfma((R)b[13], x3.e[i], rfma((R)b[11], x2.e[i], scale(x1.e[i], (R)b[9])));
+        w.e[i] = rfma((R)b[7], x3.e[i], rfma((R)b[5], x2.e[i], scale(x1.e[i], (R)b[3])));
+        z.e[i] = rfma((R)b[12], x3.e[i], rfma((R)b[10], x2.e[i], scale(x1.e[i], (R)b[8])));
+        v.e[i] = rfma((R)b[6], x3.e[i], rfma((R)b[4], x2.e[i], scale(x1.e[i], (R)b[2])));
       }
-      it.Tt[e] = t;
-      it.W[e] = w;
-      it.P3[e] = z;
-      it.V[e] = v;
+      ew_diag<W>(e, n, [&](int i, bool diag) {
+        if (diag) {
+          w.e[i] = add_real(w.e[i], (R)b[1]);
+          v.e[i] = add_real(v.e[i], (R)b[0]);
+        }
+      });
+      ew_store<W>(it.Tt + e, t);
+      ew_store<W>(it.W + e, w);
+      ew_store<W>(it.P3 + e, z);
+      ew_store<W>(it.V + e, v);
     }
-  }
+  });
 }
 
 // p = V + U over P0 (which holds U), q = V - U over V
 template <typename T, typename Wd>
 __global__ void __launch_bounds__(256) b_split_kernel(const BItem<T, Wd> *__restrict__ items) {
   const BItem<T, Wd> it = items[blockIdx.x];
-  const int nn = it.n * it.n;
-  const int end = min(nn, (int)(blockIdx.y + 1) * kEwChunk);
-  for (int e = blockIdx.y * kEwChunk + threadIdx.x; e < end; e += blockDim.x) {
-    const T u = it.P0[e], v = it.V[e];
-    it.P0[e] = add(v, u);
-    it.V[e] = sub(v, u);
-  }
+  ew_for<T>(it.V, it.n * it.n, [&](auto piece, int e) {
+    constexpr int W = decltype(piece)::value;
+    const Pack<W, T> u = ew_load<W>(it.P0 + e), v = ew_load<W>(it.V + e);
+    Pack<W, T> p, q;
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      p.e[i] = add(v.e[i], u.e[i]);
+      q.e[i] = sub(v.e[i], u.e[i]);
+    }
+    ew_store<W>(it.P0 + e, p);
+    ew_store<W>(it.V + e, q);
+  });
 }
 
 // s > 0: wa = (Wd) X, the Pade quotient
@@ -1903,66 +1978,84 @@ __global__ void __launch_bounds__(256) v_even_odd_kernel(const BVItem<T, Wd> *__
   const BVItem<T, Wd> it = items[blockIdx.x];
   const BPlan pl = plans[blockIdx.x];
   const double *b = c_pade[degree_slot(pl.m)];
-  const int n = it.n, nn = n * n;
-  const int end = min(nn, (int)(blockIdx.y + 1) * kEwChunk);
+  const int n = it.n;
   const T *P[4] = {it.P0, it.P1, it.P2, it.P3};
   const T *M[4] = {it.M0, it.M1, it.M2, it.M3};
-  for (int e = blockIdx.y * kEwChunk + threadIdx.x; e < end; e += blockDim.x) {
-    const int c = e / n, r = e - c * n;
-    const bool diag = r == c;
+  ew_for<T>(it.V, n * n, [&](auto piece, int e) {
+    constexpr int W = decltype(piece)::value;
     if (pl.m != 13) {
-      T v = elem<T>::zero(), w = elem<T>::zero(), lv = elem<T>::zero(), lw = elem<T>::zero();
+      Pack<W, T> v, w, lv, lw;
+#pragma unroll
+      for (int i = 0; i < W; ++i) v.e[i] = w.e[i] = lv.e[i] = lw.e[i] = elem<T>::zero();
       for (int k = 0; k < pl.np; ++k) {
-        const T x = P[k][e], y = M[k][e];
-        v = rfma((R)b[2 * k + 2], x, v);
-        w = rfma((R)b[2 * k + 3], x, w);
-        lv = rfma((R)b[2 * k + 2], y, lv);
-        lw = rfma((R)b[2 * k + 3], y, lw);
+        const Pack<W, T> x = ew_load<W>(P[k] + e), y = ew_load<W>(M[k] + e);
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          v.e[i] = rfma((R)b[2 * k + 2], x.e[i], v.e[i]);
+          w.e[i] = rfma((R)b[2 * k + 3], x.e[i], w.e[i]);
+          lv.e[i] = rfma((R)b[2 * k + 2], y.e[i], lv.e[i]);
+          lw.e[i] = rfma((R)b[2 * k + 3], y.e[i], lw.e[i]);
+        }
       }
-      if (diag) {
-        v = add_real(v, (R)b[0]);
-        w = add_real(w, (R)b[1]);
-      }
-      it.V[e] = v;
-      it.W[e] = w;
-      it.LV[e] = lv;
-      it.LW[e] = lw;
+      ew_diag<W>(e, n, [&](int i, bool diag) {
+        if (diag) {
+          v.e[i] = add_real(v.e[i], (R)b[0]);
+          w.e[i] = add_real(w.e[i], (R)b[1]);
+        }
+      });
+      ew_store<W>(it.V + e, v);
+      ew_store<W>(it.W + e, w);
+      ew_store<W>(it.LV + e, lv);
+      ew_store<W>(it.LW + e, lw);
     } else {
-      const T x1 = it.P0[e], x2 = it.P1[e], x3 = it.P2[e];
-      const T y1 = it.M0[e], y2 = it.M1[e], y3 = it.M2[e];
-      auto comb = [&](T a1, T a2, T a3, int i1, int i2, int i3) {
-        return rfma((R)b[i3], a3, rfma((R)b[i2], a2, scale(a1, (R)b[i1])));
+      const Pack<W, T> x1 = ew_load<W>(it.P0 + e), x2 = ew_load<W>(it.P1 + e), x3 = ew_load<W>(it.P2 + e);
+      const Pack<W, T> y1 = ew_load<W>(it.M0 + e), y2 = ew_load<W>(it.M1 + e), y3 = ew_load<W>(it.M2 + e);
+      auto comb = [&](const Pack<W, T> &a1, const Pack<W, T> &a2, const Pack<W, T> &a3, int i1, int i2, int i3) {
+        Pack<W, T> o;
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+          o.e[i] = rfma((R)b[i3], a3.e[i], rfma((R)b[i2], a2.e[i], scale(a1.e[i], (R)b[i1])));
+        return o;
       };
-      T w = comb(x1, x2, x3, 3, 5, 7), v = comb(x1, x2, x3, 2, 4, 6);
-      if (diag) {
-        w = add_real(w, (R)b[1]);
-        v = add_real(v, (R)b[0]);
-      }
-      it.T1[e] = comb(x1, x2, x3, 9, 11, 13);
-      it.W[e] = w;
-      it.P3[e] = comb(x1, x2, x3, 8, 10, 12);
-      it.V[e] = v;
-      it.T2[e] = comb(y1, y2, y3, 9, 11, 13);
-      it.LW[e] = comb(y1, y2, y3, 3, 5, 7);
-      it.M3[e] = comb(y1, y2, y3, 8, 10, 12);
-      it.LV[e] = comb(y1, y2, y3, 2, 4, 6);
+      Pack<W, T> w = comb(x1, x2, x3, 3, 5, 7), v = comb(x1, x2, x3, 2, 4, 6);
+      ew_diag<W>(e, n, [&](int i, bool diag) {
+        if (diag) {
+          w.e[i] = add_real(w.e[i], (R)b[1]);
+          v.e[i] = add_real(v.e[i], (R)b[0]);
+        }
+      });
+      ew_store<W>(it.T1 + e, comb(x1, x2, x3, 9, 11, 13));
+      ew_store<W>(it.W + e, w);
+      ew_store<W>(it.P3 + e, comb(x1, x2, x3, 8, 10, 12));
+      ew_store<W>(it.V + e, v);
+      ew_store<W>(it.T2 + e, comb(y1, y2, y3, 9, 11, 13));
+      ew_store<W>(it.LW + e, comb(y1, y2, y3, 3, 5, 7));
+      ew_store<W>(it.M3 + e, comb(y1, y2, y3, 8, 10, 12));
+      ew_store<W>(it.LV + e, comb(y1, y2, y3, 2, 4, 6));
     }
-  }
+  });
 }
 
 // p = V + U over T1, q = V - U over V; dp = dV + dU over T2, dq = dV - dU over LV
 template <typename T, typename Wd>
 __global__ void __launch_bounds__(256) v_split_kernel(const BVItem<T, Wd> *__restrict__ items) {
   const BVItem<T, Wd> it = items[blockIdx.x];
-  const int nn = it.n * it.n;
-  const int end = min(nn, (int)(blockIdx.y + 1) * kEwChunk);
-  for (int e = blockIdx.y * kEwChunk + threadIdx.x; e < end; e += blockDim.x) {
-    const T u = it.T1[e], v = it.V[e], du = it.T2[e], dv = it.LV[e];
-    it.T1[e] = add(v, u);
-    it.V[e] = sub(v, u);
-    it.T2[e] = add(dv, du);
-    it.LV[e] = sub(dv, du);
-  }
+  auto split = [](T *u, T *v, int n) {  // (u, v) <- (v + u, v - u)
+    ew_for<T>(u, n * n, [&](auto piece, int e) {
+      constexpr int W = decltype(piece)::value;
+      const Pack<W, T> a = ew_load<W>(u + e), c = ew_load<W>(v + e);
+      Pack<W, T> p, q;
+#pragma unroll
+      for (int i = 0; i < W; ++i) {
+        p.e[i] = add(c.e[i], a.e[i]);
+        q.e[i] = sub(c.e[i], a.e[i]);
+      }
+      ew_store<W>(u + e, p);
+      ew_store<W>(v + e, q);
+    });
+  };
+  split(it.T1, it.V, it.n);
+  split(it.T2, it.LV, it.n);
 }
 
 // s > 0: (wr, wl) = wide (R, dR)
