@@ -4,8 +4,10 @@
 // WarpWraps: src/expm/pade.cppm:186-188).
 //
 // Blocked right-looking factorisation, panel width kb <= 64:
-//   1. panel: one thread-block CLUSTER (<= 8 CTAs) holds the h x kb panel in
-//      the CTAs' shared memory, rows split across the CTAs. Per pivot column:
+//   1. panel: heights up to 4096 in lu_panel.cuh (one row per thread, a cluster
+//      of eight CTAs); taller ones in lu_panel_kernel below, whose cluster
+//      (<= 8 CTAs) holds the h x kb panel in the CTAs' shared memory. Per pivot
+//      column there:
 //        - every CTA reduces its local pivot candidate (largest |Re|+|Im|,
 //          first index on ties -- LAPACK IxAMAX) and publishes it, with the
 //          candidate's whole row, into a double-buffered slot;
@@ -19,11 +21,13 @@
 //      That is two CTA barriers and one cluster barrier per column.
 //   2. swap + TRSM: one warp per column outside the panel applies the panel's
 //      row permutation (a compact gather of <= 2 kb rows) and, right of the
-//      panel, solves with the unit-lower L11 held in shared memory.
+//      panel and in a right-hand side, solves with the unit-lower L11 held in
+//      shared memory.
 //   3. trailing update: A22 -= L21 U12 on the tensor-core GEMM.
-// The solve gathers the right-hand side through the accumulated row
-// permutation and runs blocked forward / backward substitution (diagonal
-// blocks per warp, off-diagonal blocks on the GEMM).
+// getrf_solve runs the forward substitution of its right-hand side beside the
+// factorisation, then blocked backward substitution (diagonal blocks per warp,
+// off-diagonal blocks on the GEMM); getrs gathers the right-hand side through
+// the accumulated row permutation and runs both.
 #include <cooperative_groups.h>
 #include <climits>
 #include <type_traits>
@@ -69,8 +73,7 @@ __host__ __device__ inline std::size_t align16(std::size_t x) { return (x + 15) 
 
 // Offsets of the panel kernel's shared-memory regions (host and device agree).
 struct PanelSmem {
-  std::size_t S, slot_row, slot_diag, cand, oldrow, slot_rcp, cand_rcp, slot_val, slot_idx,
-      cand_val, cand_idx, red_val, red_idx, plist, flags, map_pos, map_org, total;
+  std::size_t S, slot_row, slot_diag, cand, oldrow, slot_val, slot_idx, cand_val, cand_idx, red_val, red_idx, plist, flags, map_pos, map_org, total;
 };
 template <typename T>
 __host__ __device__ inline PanelSmem panel_smem(int rpc, int kb) {
@@ -81,8 +84,6 @@ __host__ __device__ inline PanelSmem panel_smem(int rpc, int kb) {
   o.slot_diag = at; at = align16(at + sizeof(T) * 2 * kb);
   o.cand = at; at = align16(at + sizeof(T) * kMaxCluster * kb);
   o.oldrow = at; at = align16(at + sizeof(T) * kb);
-  o.slot_rcp = at; at = align16(at + sizeof(T) * 2);
-  o.cand_rcp = at; at = align16(at + sizeof(T) * kMaxCluster);
   o.slot_val = at; at = align16(at + sizeof(double) * 2);
   o.slot_idx = at; at = align16(at + sizeof(int) * 2);
   o.cand_val = at; at = align16(at + sizeof(double) * kMaxCluster);
@@ -333,7 +334,7 @@ __global__ void __launch_bounds__(kPanelThreads)
                g_map_count, info);
 }
 
-// Epilogue shared by both panel kernels: the pivot vector, LAPACK's info, the
+// Epilogue of the panel kernel: the pivot vector, LAPACK's info, the
 // compact row map the swap kernel replays, and the accumulated permutation.
 // Ends with the cluster barrier that keeps every CTA's shared memory alive
 // until the last remote read of it has completed.
