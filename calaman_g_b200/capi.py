@@ -132,6 +132,8 @@ for _suf, _real in (("s", c_float), ("d", c_double), ("c", c_float), ("z", c_dou
     SIGNATURES[f"calaman_gemm_{_suf}"] = (Status, _GEMM)
     SIGNATURES[f"calaman_getrf_{_suf}"] = (Status, [c_void_p, c_int, c_void_p, c_int, c_void_p,
                                                    c_int_p])
+    SIGNATURES[f"calaman_getrf_wait_check_{_suf}"] = (Status, [c_void_p, c_int, c_void_p, c_int, c_void_p,
+                                                              c_int, c_int, c_int_p])
     SIGNATURES[f"calaman_getrs_{_suf}"] = (Status, [c_void_p, c_int, c_int, c_void_p, c_int,
                                                    c_void_p, c_void_p, c_int, c_void_p, c_int,
                                                    c_int_p])

@@ -813,6 +813,16 @@ calamanStatus_t calaman_getrf_bufferSize(int n, size_t *bytes) {
                       scratch, d_info));                                                       \
     return ok_status();                                                                        \
   }                                                                                            \
+  calamanStatus_t calaman_getrf_wait_check_##SUF(calamanStream_t stream, int n, PT A, int lda, \
+                                                 void *scratch, int drop_from,                 \
+                                                 int tries, int *d_info) {                     \
+    if (n < 1 || n > kMaxDim || lda < n || A == nullptr || scratch == nullptr ||               \
+        drop_from < 0 || tries < 0 || d_info == nullptr)                                       \
+      return blas_status(CALAMAN_STATUS_INVALID_VALUE);                                        \
+    CLM_CUDA(getrf<T>(static_cast<cudaStream_t>(stream), n, reinterpret_cast<T *>(A), lda,     \
+                      scratch, d_info, PanelWait{tries, drop_from}));                          \
+    return ok_status();                                                                        \
+  }                                                                                            \
   calamanStatus_t calaman_getrs_##SUF(calamanStream_t stream, int n, int nrhs, CPT LU,         \
                                       int lda, const void *scratch, CPT B, int ldb, PT X,      \
                                       int ldx, int *d_info) {                                  \

@@ -4,6 +4,8 @@
 // never synchronises. Matrices are column-major.
 #pragma once
 
+#include <climits>
+
 #include "common.cuh"
 
 namespace clm {
@@ -97,10 +99,19 @@ cudaError_t oz_gemm(cudaStream_t s, int M, int N, int K, double alpha, const T *
 // small swap map; bytes for an n x n factorisation.
 std::size_t lu_scratch_bytes(int n);
 
+// The bounded waits of the panels (lu_panel.cuh). Normal use: the defaults, every
+// CTA pushes in every column. Self-test: from panel column drop_from on, the last
+// CTA of a cluster pushes nothing, so that waits run out after `tries`.
+struct PanelWait {
+  int tries = 1 << 20;
+  int drop_from = INT_MAX;
+};
+
 // Factor A (n x n, lda) in place: P A = L U. info_dev[0] receives the first
-// zero pivot (1-based) or 0. `scratch` is lu_scratch_bytes(n) device bytes.
+// zero pivot (1-based), 0, or n + 1 if a panel's wait ran out (A is then not
+// factored). `scratch` is lu_scratch_bytes(n) device bytes.
 template <typename T>
-cudaError_t getrf(cudaStream_t s, int n, T *A, int lda, void *scratch, int *info_dev);
+cudaError_t getrf(cudaStream_t s, int n, T *A, int lda, void *scratch, int *info_dev, PanelWait wait = {});
 
 // While a NoLookAheadScope is open on a host thread, getrf on that thread
 // factors every panel on the caller's stream instead of overlapping the next

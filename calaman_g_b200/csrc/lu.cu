@@ -660,7 +660,7 @@ inline cudaLaunchAttribute cluster_attr(int ncta) {
 // four CTAs, 1.37 on eight).
 template <typename T, int KB, int MAXT>
 cudaError_t launch_rows_panel(cudaStream_t s, int n, T *A, int lda, int k, int kb, const LuScratch &sc,
-                              const RowMap &map, int *info) {
+                              const RowMap &map, int *info, const PanelWait &wait) {
   const int h = n - k;
   const int ncta = h <= MAXT ? 1 : kPanelMaxCluster;
   int nt = ((h + ncta - 1) / ncta + 31) / 32 * 32;
@@ -678,16 +678,16 @@ cudaError_t launch_rows_panel(cudaStream_t s, int n, T *A, int lda, int k, int k
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   note_launch();
-  return cudaLaunchKernelEx(&cfg, kern, n, A, lda, k, kb, sc.ipiv, sc.perm, map.pos, map.src, map.count, info);
+  return cudaLaunchKernelEx(&cfg, kern, n, A, lda, k, kb, sc.ipiv, sc.perm, map.pos, map.src, map.count, info, wait);
 }
 
 template <typename T>
 cudaError_t launch_panel(cudaStream_t s, int n, T *A, int lda, int k, int kb, const LuScratch &sc,
-                         const RowMap &map, int *info) {
+                         const RowMap &map, int *info, const PanelWait &wait) {
   const int h = n - k;
   using C = RowsPanel<T>;
-  if (n <= short_rows<T>()) return launch_rows_panel<T, C::KBs, C::MAXTs>(s, n, A, lda, k, kb, sc, map, info);
-  if (h <= kRowsMax) return launch_rows_panel<T, C::KB, C::MAXT>(s, n, A, lda, k, kb, sc, map, info);
+  if (n <= short_rows<T>()) return launch_rows_panel<T, C::KBs, C::MAXTs>(s, n, A, lda, k, kb, sc, map, info, wait);
+  if (h <= kRowsMax) return launch_rows_panel<T, C::KB, C::MAXT>(s, n, A, lda, k, kb, sc, map, info, wait);
   // enough CTAs for the panel to fit, and for every row to get >= 2 lanes of
   // the fused pass when the cluster allows it (<= 256 rows per CTA)
   int ncta = (int)(((std::size_t)h * kb * sizeof(T) + kPanelSmemBudget - 1) / kPanelSmemBudget);
@@ -787,7 +787,7 @@ cudaError_t lookahead(LookAhead *&out) {
 // 12918 (with the split inside its updates), complex64 777 3123 -> 2591.
 template <typename T>
 static cudaError_t factor(cudaStream_t s, int n, T *A, int lda, const LuScratch &sc, int *info_dev, bool keep_l,
-                          int nrhs, T *B, int ldb, T *X, int ldx) {
+                          int nrhs, T *B, int ldb, T *X, int ldx, const PanelWait &wait = {}) {
   cudaError_t e = cudaMemsetAsync(info_dev, 0, sizeof(int), s);
   if (e != cudaSuccess) return e;
   iota_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, sc.perm);
@@ -803,7 +803,7 @@ static cudaError_t factor(cudaStream_t s, int n, T *A, int lda, const LuScratch 
   const bool ahead = n > kbn && !tl_no_lookahead;
   LookAhead *la = nullptr;
   if (ahead && (e = lookahead(la)) != cudaSuccess) return e;
-  if ((e = launch_panel<T>(s, n, A, lda, 0, kbn < n ? kbn : n, sc, sc.map[0], info_dev)) != cudaSuccess) return e;
+  if ((e = launch_panel<T>(s, n, A, lda, 0, kbn < n ? kbn : n, sc, sc.map[0], info_dev, wait)) != cudaSuccess) return e;
   for (int k = 0, step = 0; k < n; k += kbn, ++step) {
     const int kb = (k + kbn < n) ? kbn : n - k;
     const RowMap &map = sc.map[step & 1];
@@ -831,10 +831,11 @@ static cudaError_t factor(cudaStream_t s, int n, T *A, int lda, const LuScratch 
       if (ahead) {
         if ((e = cudaEventRecord(la->ready, s)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(la->aux, la->ready, 0)) != cudaSuccess) return e;
-        if ((e = launch_panel<T>(la->aux, n, A, lda, k + kb, kb2, sc, sc.map[(step + 1) & 1], info_dev)) != cudaSuccess)
+        if ((e = launch_panel<T>(la->aux, n, A, lda, k + kb, kb2, sc, sc.map[(step + 1) & 1], info_dev, wait)) !=
+            cudaSuccess)
           return e;
         if ((e = cudaEventRecord(la->done, la->aux)) != cudaSuccess) return e;
-      } else if ((e = launch_panel<T>(s, n, A, lda, k + kb, kb2, sc, sc.map[(step + 1) & 1], info_dev)) !=
+      } else if ((e = launch_panel<T>(s, n, A, lda, k + kb, kb2, sc, sc.map[(step + 1) & 1], info_dev, wait)) !=
                  cudaSuccess) {  // disjoint from the other columns
         return e;
       }
@@ -850,9 +851,9 @@ static cudaError_t factor(cudaStream_t s, int n, T *A, int lda, const LuScratch 
 }
 
 template <typename T>
-cudaError_t getrf(cudaStream_t s, int n, T *A, int lda, void *scratch, int *info_dev) {
+cudaError_t getrf(cudaStream_t s, int n, T *A, int lda, void *scratch, int *info_dev, PanelWait wait) {
   if (n < 1) return cudaSuccess;
-  return factor<T>(s, n, A, lda, carve_lu(scratch, n), info_dev, true, 0, nullptr, 0, nullptr, 0);
+  return factor<T>(s, n, A, lda, carve_lu(scratch, n), info_dev, true, 0, nullptr, 0, nullptr, 0, wait);
 }
 
 // X <- L^-1 X (lower) and X <- U^-1 X (upper) by diagonal blocks.
@@ -931,7 +932,7 @@ cudaError_t getrs(cudaStream_t s, int n, int nrhs, const T *LU, int lda, const v
 }
 
 #define CLM_INST_LU(T)                                                                            \
-  template cudaError_t getrf<T>(cudaStream_t, int, T *, int, void *, int *);                     \
+  template cudaError_t getrf<T>(cudaStream_t, int, T *, int, void *, int *, PanelWait);          \
   template cudaError_t getrs<T>(cudaStream_t, int, int, const T *, int, const void *, const T *, \
                                 int, T *, int, int *);                                           \
   template cudaError_t getrf_solve<T>(cudaStream_t, int, T *, int, void *, int, T *, int, T *, int, bool, int *);

@@ -101,6 +101,9 @@ struct alignas(16) PivotSlot {
 
 constexpr int kPanelMaxCluster = 8;
 
+constexpr unsigned kGaveUp = 0xffffffffu;  // above the key of every candidate
+constexpr long long kPanelDrainTries = 1ll << 12;  // for pushes under way when a panel is given up
+
 // Bytes of dynamic shared memory the kernel below takes with nt threads.
 template <typename T, int KB>
 inline std::size_t panel_rows_smem(int nt) { return sizeof(T) * (std::size_t)KB * nt; }
@@ -124,13 +127,19 @@ inline std::size_t panel_rows_smem(int nt) { return sizeof(T) * (std::size_t)KB 
 // every CTA's push for column j + 1, which each CTA issues after a barrier
 // behind its last read of column j.
 //
-// Bound: the latency of that chain, once per column. Waits are bounded; one
-// that runs out sets info = n + 1 and no later wait is made.
+// Bound: the latency of that chain, once per column. Waits are bounded. A warp
+// whose wait runs out uses nothing of the slots; in the place of its candidate for
+// the next column it leaves a key above all others, at which its whole CTA leaves
+// the loop, and it raises a flag in every CTA, read behind the cluster barrier at
+// the end. Permutation and map are written only if no CTA gave up. Otherwise the
+// panel's rows are in no defined order, its pivots and its map are the identity
+// (what runs behind it stays in range), info = n + 1, and every CTA waits once
+// more, bounded, for pushes under way to it.
 template <typename T, int KB, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1)
     lu_panel_rows_kernel(int n, T *__restrict__ A, int lda, int k, int kb, int *__restrict__ ipiv,
                          int *__restrict__ perm, int *__restrict__ g_map_pos, int *__restrict__ g_map_src,
-                         int *__restrict__ g_map_count, int *__restrict__ info) {
+                         int *__restrict__ g_map_count, int *__restrict__ info, const PanelWait wait) {
   namespace cgr = cooperative_groups;
   constexpr int U = 8;                    // places per guarded group of the update
   constexpr int V = 16 / (int)sizeof(T);  // elements per 16-byte piece
@@ -154,8 +163,10 @@ __global__ void __launch_bounds__(MAXT, 1)
   __shared__ int wpos[2][MAXT / 32];
   __shared__ __align__(8) uint64_t bar[2];
   __shared__ int below[2];
+  __shared__ int failed;  // a warp of any CTA gave up
 
   if (tid == 0) {
+    failed = 0;
     tc::mbar_init(&bar[0], 1);
     tc::mbar_init(&bar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -163,9 +174,9 @@ __global__ void __launch_bounds__(MAXT, 1)
   T r[KB];
 #pragma unroll
   for (int c = 0; c < KB; ++c) r[c] = (has && c < kb) ? P[(std::size_t)c * lda + gi] : elem<T>::zero();
-  if (ncta > 1) cluster.sync();  // the mbarriers exist before any push
+  if (ncta > 1) cluster.sync();  // the mbarriers and the flag exist before any push
 
-  bool active = has, gave_up = false;
+  bool active = has;
   int pos = gi, own = kb, first_zero = -1;  // own: the step at which this row became the pivot
   auto warp_candidate = [&](int buf) {
     const PivotCand c = warp_best<T>(pivot_cand<T>(r[0], pos, active));
@@ -176,8 +187,9 @@ __global__ void __launch_bounds__(MAXT, 1)
     }
   };
   warp_candidate(0);
+  int j = 0;
 #pragma unroll 1
-  for (int j = 0; j < kb; ++j) {
+  for (; j < kb; ++j) {
     const int par = j & 1;
     const int live = KB - j;                          // places that hold columns of the panel
     const int pieces = (live + U - 1) / U * (U / V);  // 16-byte pieces of the row that still matter
@@ -190,6 +202,7 @@ __global__ void __launch_bounds__(MAXT, 1)
     if constexpr (!std::is_same<T, float>::value) c.lo = lane < nwarps ? wkey[par][1][lane] : 0u;
     c.pos = lane < nwarps ? wpos[par][lane] : INT_MAX;
     c = warp_best<T>(c);
+    if (ncta > 1 && c.hi == kGaveUp) break;
     const bool mine = active && pos == c.pos;
     // the winner's warp publishes it; a CTA without candidates publishes that
     if (__any_sync(0xffffffffu, mine) || (c.pos == INT_MAX && warp == 0)) {
@@ -212,7 +225,7 @@ __global__ void __launch_bounds__(MAXT, 1)
         }
         out->rcp[0] = zero ? elem<T>::one() : divide(elem<T>::one(), r[0]);
       }
-      if (ncta > 1) {
+      if (ncta > 1 && (j < wait.drop_from || rank + 1 < ncta)) {
         __syncwarp();
         for (int t = lane; t < (kHead + pieces) << lg; t += 32) {
           const int q = t & (ncta - 1), at = t >> lg;
@@ -223,12 +236,19 @@ __global__ void __launch_bounds__(MAXT, 1)
     }
     int from = 0;
     if (ncta > 1) {
-      if (!gave_up && !tc::mbar_wait(&bar[par], (unsigned)(j >> 1) & 1u, 1ll << 20)) gave_up = true;
+      bool arrived = false;
+      for (int i = 0; i < wait.tries && !arrived; ++i) arrived = tc::mbar_try_wait(&bar[par], (unsigned)(j >> 1) & 1u);
       c.hi = lane < ncta ? slot[par][lane].hi : 0u;
       c.lo = lane < ncta ? slot[par][lane].lo : 0u;
       const int p = lane < ncta ? slot[par][lane].pos : INT_MAX;
       c.pos = p;
+      const bool all = __all_sync(0xffffffffu, arrived);
       c = warp_best<T>(c);
+      if (!all) {  // the slots say nothing
+        if (lane == 0) wkey[par ^ 1][0][warp] = kGaveUp;
+        if (lane < ncta) *cluster.map_shared_rank(&failed, lane) = 1;
+        continue;
+      }
       from = __ffs(__ballot_sync(0xffffffffu, p == c.pos)) - 1;
     } else {
       __syncthreads();
@@ -290,8 +310,22 @@ __global__ void __launch_bounds__(MAXT, 1)
   const bool down = has && gi < kb && pos >= kb;
   const unsigned downs = __ballot_sync(0xffffffffu, down);
   if (rank == 0 && warp < 2 && lane == 0) below[warp] = __popc(downs);
-  if (ncta > 1) cluster.sync();  // every read of perm is done
+  if (ncta > 1) cluster.sync();  // every read of perm is done, every flag is there
   else __syncthreads();
+  if (failed) {
+    if (rank == 0 && tid < kb) {  // at least 64 threads
+      ipiv[k + tid] = k + tid;
+      g_map_pos[tid] = g_map_src[tid] = k + tid;
+      if (tid == 0) {
+        *g_map_count = kb;
+        info[0] = n + 1;
+      }
+    }
+    // the column given up and the one behind it, which a peer may have entered
+    if (ncta > 1 && tid == 0)
+      for (int c = j - 1; c <= j; ++c) tc::mbar_wait(&bar[c & 1], (unsigned)(c >> 1) & 1u, kPanelDrainTries);
+    return;
+  }
   if (moved) perm[k + pos] = old;
   if (has && pos < kb) {
     g_map_pos[pos] = k + pos;
@@ -306,7 +340,6 @@ __global__ void __launch_bounds__(MAXT, 1)
     *g_map_count = kb + below[0] + (nwarps > 1 ? below[1] : 0);
     if (first_zero >= 0 && info[0] == 0) info[0] = k + first_zero + 1;
   }
-  if (gave_up) info[0] = n + 1;
 }
 
 }  // namespace clm

@@ -120,8 +120,9 @@ calamanStatus_t calaman_pade_bufferSize_z(calamanSolverHandle_t h, int m, int n,
 
 /* ---- expm (src/expm/expm.cppm:87-174) ----------------------------------
  * exp(A) by scaling and squaring with a diagonal Pade approximant (Higham
- * 2005, Algorithm 2.3). d_info: device array of 2 ints ([0] LU info, [1]
- * solve info). plan may be NULL. Synchronises `stream` once.
+ * 2005, Algorithm 2.3). d_info: device array of 2 ints ([0] LU info as getrf's
+ * below: the first zero pivot, 0, or n + 1 if a bounded wait ran out and d_expA is
+ * not defined; [1] solve info). plan may be NULL. Synchronises `stream` once.
  * The _s/_c tiers run their dense products as split-BF16 tensor-core GEMMs
  * with FP32 accumulation; the 1-norm is always accumulated in FP64. */
 calamanStatus_t calaman_expm_s(calamanBlasHandle_t blas, calamanSolverHandle_t solver,
@@ -386,7 +387,7 @@ calamanStatus_t calaman_expm_noalloc_d(calamanBlasHandle_t blas, calamanStream_t
                                        int *d_info, calamanExpmPlan_t *plan);
 
 /* ---- pade (src/expm/pade.cppm:77-191) ----------------------------------
- * Unscaled r_m(A) = q_m(A)^-1 p_m(A); never synchronises. */
+ * Unscaled r_m(A) = q_m(A)^-1 p_m(A); never synchronises. d_info as expm's. */
 calamanStatus_t calaman_pade_s(calamanBlasHandle_t blas, calamanSolverHandle_t solver,
                                calamanStream_t stream, int m, int n, const float *d_A, int lda,
                                float *d_r, int ldr, void *d_work, size_t lwork_bytes, int *d_info);
@@ -582,7 +583,9 @@ calamanStatus_t calaman_grid_barrier_wait_check(calamanStream_t stream, unsigned
  * = first entry of largest |Re|+|Im|. `scratch` is calaman_getrf_bufferSize
  * device bytes; it begins with the n pivot rows (0-based, int) and must be
  * passed unchanged to getrs. getrs reads B and writes X (no aliasing).
- * d_info: getrf writes the first zero pivot (1-based) or 0; getrs writes 0. */
+ * d_info: getrf writes the first zero pivot (1-based), 0, or n + 1 if a bounded
+ * wait between the thread blocks of a panel ran out (A is then not factored and
+ * the solve's result not defined; every pivot is in range); getrs writes 0. */
 calamanStatus_t calaman_getrf_bufferSize(int n, size_t *bytes);
 calamanStatus_t calaman_getrf_s(calamanStream_t stream, int n, float *A, int lda, void *scratch,
                                 int *d_info);
@@ -604,6 +607,18 @@ calamanStatus_t calaman_getrs_c(calamanStream_t stream, int n, int nrhs, const v
 calamanStatus_t calaman_getrs_z(calamanStream_t stream, int n, int nrhs, const void *LU, int lda,
                                 const void *scratch, const void *B, int ldb, void *X, int ldx,
                                 int *d_info);
+/* Self-test of those waits: getrf whose panels of more than one thread block
+ * push nothing from the last block from panel column drop_from on, each wait
+ * limited to `tries` tries (0: every wait runs out at once). n + 1 in d_info says
+ * that a panel gave up. Never synchronises. No counterpart in the reference. */
+calamanStatus_t calaman_getrf_wait_check_s(calamanStream_t stream, int n, float *A, int lda, void *scratch,
+                                           int drop_from, int tries, int *d_info);
+calamanStatus_t calaman_getrf_wait_check_d(calamanStream_t stream, int n, double *A, int lda, void *scratch,
+                                           int drop_from, int tries, int *d_info);
+calamanStatus_t calaman_getrf_wait_check_c(calamanStream_t stream, int n, void *A, int lda, void *scratch,
+                                           int drop_from, int tries, int *d_info);
+calamanStatus_t calaman_getrf_wait_check_z(calamanStream_t stream, int n, void *A, int lda, void *scratch,
+                                           int drop_from, int tries, int *d_info);
 
 /* Total kernel launches this library has issued in the process. */
 unsigned long long calamanGetLaunchCount(void);

@@ -198,3 +198,40 @@ def test_getrf_nan_column_keeps_its_row(lib, oracle, n):
     _, _, _, ipiv, info = run_getrf(lib, a, "d")
     _, opiv, _ = oracle.getrf(a)
     assert np.array_equal(ipiv[:41], opiv[:41]) and ipiv[40] == 40
+
+
+@pytest.mark.parametrize("suf,n,lda", [("s", 1300, 1303), ("d", 900, 900), ("c", 700, 701), ("z", 2100, 2100),
+                                       ("d", 400, 400)])
+@pytest.mark.parametrize("drop,tries", [(0, 1 << 12), (3, 1 << 12), (5, 0)])
+def test_panel_waits_run_out_in_range(lib, oracle, suf, n, lda, drop, tries):
+    """From panel column `drop` on one CTA of a panel pushes nothing (tries = 0: no wait lasts): every CTA gives
+    the panel up with the same outcome. info is n + 1, the pivots are in range, the padding rows, the scratch's
+    end and the bytes behind the matrix are untouched, and the next call is right.
+    A panel on one CTA (n = 400) has no such wait."""
+    import torch
+
+    a = gaussian(n, suf, 940 + n)
+    guard = 4096
+    buf = np.concatenate([colmajor_buffer(a, lda, suf), np.full(guard, 7, dtype=NP_DTYPE[suf])])
+    dA = torch.from_numpy(buf).cuda()
+    b = ctypes.c_size_t()
+    assert lib.calaman_getrf_bufferSize(n, ctypes.byref(b)).ok
+    scratch = torch.full((b.value + guard,), 0x5A, dtype=torch.uint8, device="cuda")
+    info = torch.full((2,), -5, dtype=torch.int32, device="cuda")
+    ip = ctypes.cast(info.data_ptr(), ctypes.POINTER(ctypes.c_int))
+    st = getattr(lib, f"calaman_getrf_wait_check_{suf}")(None, n, vp(dA), lda, vp(scratch), drop, tries, ip)
+    torch.cuda.synchronize()
+    assert st.ok, st
+    got = dA.cpu().numpy()
+    ipiv = scratch[: 4 * n].view(torch.int32).cpu().numpy()
+    one_cta = n <= 512
+    assert info.tolist() == [0 if one_cta else n + 1, -5]
+    if not one_cta:
+        assert np.array_equal(ipiv, np.arange(n))
+    assert bool((scratch[b.value:] == 0x5A).all())
+    assert np.array_equal(got[n * lda:], buf[n * lda:])
+    assert np.array_equal(got[: n * lda].reshape(n, lda)[:, n:], buf[: n * lda].reshape(n, lda)[:, n:])
+    _, _, lu, ipiv, again = run_getrf(lib, a, suf)
+    assert again == 0 and np.isfinite(lu).all()
+    if suf in "dz" and n < 1000:
+        assert np.array_equal(ipiv, oracle.getrf(a)[1])
