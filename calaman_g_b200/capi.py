@@ -158,6 +158,8 @@ SIGNATURES["calamanGetDoubleEmulation"] = (Status, [_H, c_int_p])
 SIGNATURES["calaman_gemm_ozaki_bufferSize"] = (Status, [c_int, c_int, c_int, c_int, c_int, c_size_t_p])
 SIGNATURES["calaman_gemm_ozaki_d"] = (Status, _GEMM + [c_int, c_void_p, c_size_t])
 SIGNATURES["calaman_gemm_ozaki_z"] = (Status, _GEMM + [c_int, c_void_p, c_size_t])
+SIGNATURES["calaman_gemm_bf16x_wait_check"] = (Status, [c_void_p, ctypes.c_longlong, c_void_p, c_size_t,
+                                                        c_int_p])
 SIGNATURES["calaman_gemm_ozaki_wait_check"] = (Status, [c_void_p, ctypes.c_longlong, c_void_p, c_size_t,
                                                         c_int_p])
 SIGNATURES["calaman_expm_noalloc_d"] = (Status, [_H, c_void_p, c_int, c_void_p, c_int, c_void_p,

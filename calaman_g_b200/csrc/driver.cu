@@ -760,6 +760,23 @@ calamanStatus_t calaman_gemm_ozaki_wait_check(calamanStream_t stream, long long 
   return ok_status();
 }
 
+calamanStatus_t calaman_gemm_bf16x_wait_check(calamanStream_t stream, long long spin, void *work, size_t work_bytes,
+                                              int *code) {
+  constexpr int n = 192, k = 128;  // two k-blocks, ragged tiles
+  const std::size_t ws = align_up(tc_gemm_workspace_bytes(n, n, k, 6), 256);
+  if (work == nullptr || code == nullptr || spin < 1) return blas_status(CALAMAN_STATUS_INVALID_VALUE);
+  if (work_bytes < ws + sizeof(float) * (2 * n * k + n * n)) return blas_status(CALAMAN_STATUS_ALLOC_FAILED);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  float *A = reinterpret_cast<float *>(static_cast<char *>(work) + ws), *B = A + n * k, *C = B + n * k;
+  CLM_CUDA(cudaMemsetAsync(work, 0, sizeof(int), st));
+  CLM_CUDA(tc_gemm_f32(st, n, n, k, 1.0, A, n, B, k, 1.0, C, n, work, ws, 6, spin, /*skip=*/1));
+  int h = 0;
+  CLM_CUDA(cudaMemcpyAsync(&h, work, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CLM_CUDA(cudaStreamSynchronize(st));
+  *code = h;
+  return ok_status();
+}
+
 calamanStatus_t calaman_gemm_bf16x_bufferSize_c(int m, int n, int k, int terms, size_t *bytes) {
   if (m < 1 || n < 1 || k < 1 || (terms != 3 && terms != 6) || bytes == nullptr)
     return blas_status(CALAMAN_STATUS_INVALID_VALUE);

@@ -71,11 +71,13 @@ cudaError_t gemm_nn_splitk(cudaStream_t s, int M, int N, int K, double alpha, co
 
 // FP32 / complex64 GEMM on the tcgen05 tensor cores as split-BF16 part
 // products (terms = 3 or 6), accumulated in FP32 TMEM; needs
-// tc_gemm_workspace_bytes of scratch (cplx: for the complex product).
+// tc_gemm_workspace_bytes of scratch (cplx: for the complex product). spin, skip:
+// of the kernel for shallow products, as oz_gemm's spin and skip_loads below (skip:
+// no product is issued).
 std::size_t tc_gemm_workspace_bytes(int M, int N, int K, int terms, bool cplx = false);
 cudaError_t tc_gemm_f32(cudaStream_t s, int M, int N, int K, double alpha, const float *A, int lda,
                         const float *B, int ldb, double beta, float *C, int ldc, void *ws,
-                        std::size_t ws_bytes, int terms);
+                        std::size_t ws_bytes, int terms, long long spin = 0, int skip = 0);
 cudaError_t tc_gemm_c64(cudaStream_t s, int M, int N, int K, double alpha, const float2 *A, int lda,
                         const float2 *B, int ldb, double beta, float2 *C, int ldc, void *ws,
                         std::size_t ws_bytes, int terms);

@@ -313,10 +313,15 @@ __global__ void __launch_bounds__(256)
 // trailing updates and the updates of the triangular solves). Such a product is
 // bound by its passes over C, so the operands are split where they are used and
 // never written out as parts: one CTA per 128 x 128 tile of C, eight warps that
-// first put the loads of their old C values in flight, then read the FP32
-// operands, split them and store the part tiles K-major and 128-byte swizzled;
-// one thread issues the part products (128 x 128 x 16), the eight warps drain
-// the accumulator. 96 KB of part tiles, two CTAs per SM.
+// read the FP32 operands, split them and store the part tiles K-major and
+// 128-byte swizzled; one thread issues the part products (128 x 128 x 16), the
+// eight warps load their old C values and drain the accumulator (old C fetched
+// ahead of the products took 64 registers and spilled: 47 us against 42 at
+// 4096 x 4096 x 64). 96 KB of part tiles, two CTAs per SM.
+// The wait between the two k-blocks has one outcome for the CTA: where it runs
+// out, the part tiles are left alone, no further product is issued, C is not
+// written, and the CTA waits once more, bounded, for the products it did issue
+// before it frees its TMEM.
 // Complex64 runs as the real product of twice the rows and depth with both
 // interleaved, row 2i = Re, 2i + 1 = Im (depth alike), so that B and C are the
 // caller's arrays read as floats and only A takes the block form
@@ -335,6 +340,8 @@ struct RankParams {
   float *C;
   long long lda, ldb, ldc;  // in floats (complex: twice the caller's)
   int *err;
+  long long spin;  // tries of every wait
+  int skip;        // self-test: no product is issued, so that the waits run out
 };
 
 // One 16-byte piece (8 consecutive k of one row) of every part tile.
@@ -365,17 +372,18 @@ __global__ void __launch_bounds__(kRankThreads, 2) tc_rank_kernel(const RankPara
   }
   if (warp == 0) tmem_alloc(&tmem_slot, RN);
 
-  // old C: warp w owns rows 32 (w & 3) .. of columns 64 (w >> 2) ..
+  // C: warp w owns rows 32 (w & 3) .. of columns 64 (w >> 2) ..
   const int row = m0 + (warp & 3) * 32 + lane, col0 = n0 + (warp >> 2) * 64;
   float *const Cp = prm.C + (std::size_t)col0 * prm.ldc + row;
 
   const bool vec = (prm.ldb & 3) == 0 && (reinterpret_cast<uintptr_t>(prm.B) & 15) == 0;
   uint32_t tmem = 0;
   bool ok = true;
-  for (int kb = 0; kb < prm.nkb; ++kb) {
+  int kb = 0;
+  for (; kb < prm.nkb; ++kb) {
     if (kb > 0) {  // the part tiles are free once the products over them are done
-      ok = ok && mbar_wait(&done, (uint32_t)(kb - 1) & 1u);
-      __syncthreads();
+      ok = __syncthreads_and(mbar_wait(&done, (uint32_t)(kb - 1) & 1u, prm.spin));
+      if (!ok) break;
     }
     const int k0 = kb * TK;
     // A: lanes along the rows, eight k each
@@ -427,7 +435,7 @@ __global__ void __launch_bounds__(kRankThreads, 2) tc_rank_kernel(const RankPara
     __syncthreads();
     fence_after();
     tmem = tmem_slot;
-    if (tid == 0) {
+    if (tid == 0 && !prm.skip) {
       constexpr uint32_t idesc = idesc_bf16_f32(TM, RN);
       const uint32_t a0 = saddr(sA), b0 = saddr(sB);
       // smallest part products first: x6 (l,h) (h,l) (m,m) (m,h) (h,m) (h,h), x3 the last three
@@ -442,7 +450,8 @@ __global__ void __launch_bounds__(kRankThreads, 2) tc_rank_kernel(const RankPara
       mma_commit(&done);
     }
   }
-  ok = ok && mbar_wait(&done, (uint32_t)(prm.nkb - 1) & 1u);
+  // every product issued: kb commits were made
+  ok = mbar_wait(&done, (uint32_t)(kb - 1) & 1u, prm.spin) && ok;
   if (!ok) record_error(prm.err, 5);
   fence_after();
 #pragma unroll 1
@@ -523,7 +532,8 @@ std::size_t tc_gemm_workspace_bytes(int M, int N, int K, int terms, bool cplx) {
 namespace {
 template <typename T>
 cudaError_t tc_gemm_run(cudaStream_t s, int Mc, int N, int Kc, double alpha, const T *A, int lda, const T *B,
-                        int ldb, double beta, float *C, int ldc, void *ws, std::size_t ws_bytes, int terms) {
+                        int ldb, double beta, float *C, int ldc, void *ws, std::size_t ws_bytes, int terms,
+                        long long spin = 0, int skip = 0) {
   constexpr bool cplx = std::is_same<T, float2>::value;
   if (Mc <= 0 || N <= 0) return cudaSuccess;
   const int M = cplx ? 2 * Mc : Mc, K = cplx ? 2 * Kc : Kc;  // the real product
@@ -539,6 +549,8 @@ cudaError_t tc_gemm_run(cudaStream_t s, int Mc, int N, int Kc, double alpha, con
     const long long f = cplx ? 2 : 1;
     r.lda = f * lda, r.ldb = f * ldb, r.ldc = f * ldc;
     r.err = static_cast<int *>(ws);
+    r.spin = spin > 0 ? spin : kSpinLimit;
+    r.skip = skip;
     constexpr int smem = 6 * kPart + 1024;
     auto kern = tc_rank_kernel<cplx>;
     static bool configured = false;
@@ -605,8 +617,8 @@ cudaError_t tc_gemm_run(cudaStream_t s, int Mc, int N, int Kc, double alpha, con
 
 cudaError_t tc_gemm_f32(cudaStream_t s, int M, int N, int K, double alpha, const float *A, int lda,
                         const float *B, int ldb, double beta, float *C, int ldc, void *ws,
-                        std::size_t ws_bytes, int terms) {
-  return tc_gemm_run<float>(s, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, ws, ws_bytes, terms);
+                        std::size_t ws_bytes, int terms, long long spin, int skip) {
+  return tc_gemm_run<float>(s, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, ws, ws_bytes, terms, spin, skip);
 }
 
 cudaError_t tc_gemm_c64(cudaStream_t s, int M, int N, int K, double alpha, const float2 *A, int lda,

@@ -539,6 +539,11 @@ calamanStatus_t calaman_gemm_ozaki_z(calamanStream_t stream, int m, int n, int k
  * instead of hanging). `work`: at least 1 MiB of device memory. */
 calamanStatus_t calaman_gemm_ozaki_wait_check(calamanStream_t stream, long long spin, void *work,
                                               size_t work_bytes, int *code);
+/* The same for the split-BF16 kernel of shallow products: 192 x 192 x 128 with no
+ * product issued, so that its waits run out. `work`, at least 1 MiB, holds the
+ * scratch and behind it A, B and C, which are left as they were. */
+calamanStatus_t calaman_gemm_bf16x_wait_check(calamanStream_t stream, long long spin, void *work,
+                                              size_t work_bytes, int *code);
 
 /* The batched tier's schedule and launch mode (no counterpart: the reference
  * evaluates one matrix per call). A batched call whose configuration (sizes,

@@ -144,3 +144,26 @@ def test_complex64_alpha_beta_and_padded_lda(lib):
     ref = 0.5 * (a.astype(np.complex128) @ b.astype(np.complex128)) - 2.0 * c.astype(np.complex128)
     rel = np.linalg.norm(got - ref) / (np.linalg.norm(a) * np.linalg.norm(b) + np.linalg.norm(c))
     assert rel <= 2e-6, rel
+
+
+@pytest.mark.parametrize("spin", [1, 1 << 12])
+def test_shallow_product_waits_run_out_and_c_is_untouched(lib, spin):
+    """No product is issued: the wait between the two k-blocks runs out for the whole CTA, which leaves the
+    operands and C alone, records a code and frees its TMEM; the context then runs a correct product."""
+    import torch
+
+    nb = ctypes.c_size_t()
+    assert lib.calaman_gemm_bf16x_bufferSize(192, 192, 128, 6, ctypes.byref(nb)).ok
+    w = torch.full((1 << 20,), 0x3F, dtype=torch.uint8, device="cuda")
+    code = ctypes.c_int(-1)
+    st = lib.calaman_gemm_bf16x_wait_check(None, spin, vp(w), w.numel(), ctypes.byref(code))
+    assert st.ok, st
+    assert code.value == 5
+    assert bool((w[nb.value:] == 0x3F).all())
+    rng = np.random.default_rng(8)
+    a = rng.standard_normal((192, 128)).astype(np.float32)
+    b = rng.standard_normal((128, 192)).astype(np.float32)
+    c = rng.standard_normal((192, 192)).astype(np.float32)
+    got = run_tc(lib, a, b, c, -1.0, 1.0, 6)
+    ref = c.astype(np.float64) - a.astype(np.float64) @ b.astype(np.float64)
+    assert np.linalg.norm(got - ref) <= BOUND[6] * (np.linalg.norm(a) * np.linalg.norm(b) + np.linalg.norm(c))
