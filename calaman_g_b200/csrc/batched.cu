@@ -1053,16 +1053,13 @@ struct ExpmLu {
 
 // kFactor: LU with partial pivoting of Q, then the solve; otherwise the solve
 // alone with factors and permutation from an earlier kFactor launch.
-// kOverlap: see launch_lu (a template argument, since the extra instructions
-// alone made the FP32 kernel of a large batch 5 % slower).
-template <typename Item, typename T, typename Lu, bool kFactor, int NT, bool kOverlap>
+// kLongFirst: the matrices, sorted by ascending n, from the last on.
+template <typename Item, typename T, typename Lu, bool kFactor, int NT, bool kLongFirst>
 __global__ void __launch_bounds__(NT, BLuOcc<T, NT, Lu>::kMinBlocks)
     g_lu_kernel(const Item *__restrict__ items, const BPlan *__restrict__ plans, int *__restrict__ info,
                 int mode) {
   using R = typename elem<T>::real;
-  // the next size class may start beside this one
-  if constexpr (kOverlap) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int item = kOverlap ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+  const int item = kLongFirst ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
   const Item it = items[item];
   const BPlan pl = plans[item];
   const int n = it.n;
@@ -1309,8 +1306,6 @@ __global__ void __launch_bounds__(NT, BLuOcc<T, NT, Lu>::kMinBlocks)
     blk_rows<false, T, NT>(D, ldd, k, jb, n, n, 0, blk);
     cta_update<T, NT>(D, ldd, 0, k, 0, n, Q + (std::size_t)k * n, n, jb, blk, Ls);
   }
-  // this launch is over only when the size class before it is
-  if constexpr (kOverlap) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 template <typename T, int NT> constexpr std::size_t lu_smem_bytes() {
@@ -1321,28 +1316,23 @@ template <typename T, int NT> constexpr std::size_t lu_smem_bytes() {
 // matrices that share a CTA size: by default 64-thread CTAs for n <= 64, 128
 // for n <= 128, 256 above (small matrices pack more CTAs per SM); a schedule
 // (lu_threads[ceil(n / 16)], each >= n) may choose per size bucket.
-// A batch of few matrices (up to kOverlapItems, some two to eight CTAs per SM)
-// leaves SMs idle at the end of every launch, and the launches are of unlike
-// length: there the classes run in descending size, the longest CTAs first, each
-// launch beside the one before it (programmatic dependent launch; a launch ends
-// only after the one before, so the phases behind wait for all of them). 500
-// float64 matrices, n = 3 .. 200: 2622 -> 2226 us. Thousands of matrices fill
-// every launch nearly to its end; they keep the plain launches.
-constexpr int kOverlapItems = 8 * 148;
+// A batch of few matrices (lu_fork below) of more than one class leaves SMs idle at
+// the end of every launch, and the launches are of unlike length: there the classes
+// run beside one another, the longest CTAs first, the longest class on st and the
+// others on the forked streams.
 template <typename Item, typename T, typename Lu, bool kFactor>
 cudaError_t launch_lu(cudaStream_t st, const Item *items, const BPlan *plans, int *info, int mode,
-                      const std::vector<int> &ns, const int *lu_threads = nullptr) {
+                      const std::vector<int> &ns, LuFork *fork, const int *lu_threads = nullptr) {
   const int count = (int)ns.size();
-  const bool overlap = count <= kOverlapItems;
   auto threads_of = [&](int n) {
     const int d = n <= 64 ? 64 : n <= 128 ? 128 : 256;
     if (lu_threads == nullptr) return d;
     const int t = lu_threads[(n + 15) / 16];
     return (t == 64 || t == 128 || t == 256) && t >= n ? t : d;
   };
-  auto one = [&](auto nt_tag, auto overlap_tag, int from, int to) -> cudaError_t {
+  auto one = [&](auto nt_tag, auto long_first, cudaStream_t on, int from, int to) -> cudaError_t {
     constexpr int NT = decltype(nt_tag)::value;
-    auto kern = g_lu_kernel<Item, T, Lu, kFactor, NT, decltype(overlap_tag)::value>;
+    auto kern = g_lu_kernel<Item, T, Lu, kFactor, NT, decltype(long_first)::value>;
     constexpr std::size_t smem = lu_smem_bytes<T, NT>();
     static bool configured = false;  // once, before any graph capture of a call
     if (!configured) {
@@ -1353,39 +1343,38 @@ cudaError_t launch_lu(cudaStream_t st, const Item *items, const BPlan *plans, in
       if (e != cudaSuccess) return e;
       configured = true;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(to - from, 1, 1);
-    cfg.blockDim = dim3(NT, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = overlap && to < count ? 1 : 0;  // the first launch waits for the phases before
-    note_launch();
-    return cudaLaunchKernelEx(&cfg, kern, items + from, plans + from, info, mode);
+    kern<<<to - from, NT, smem, on>>>(items + from, plans + from, info, mode);
+    return launched();
   };
-  auto run = [&](int from, int to) -> cudaError_t {
-    auto by_size = [&](auto tag) -> cudaError_t {
-      const int nt = threads_of(ns[from]);
-      return nt == 64    ? one(std::integral_constant<int, 64>{}, tag, from, to)
-             : nt == 128 ? one(std::integral_constant<int, 128>{}, tag, from, to)
-                         : one(std::integral_constant<int, 256>{}, tag, from, to);
-    };
-    return overlap ? by_size(std::true_type{}) : by_size(std::false_type{});
+  auto run = [&](auto long_first, cudaStream_t on, int from, int to) -> cudaError_t {
+    const int nt = threads_of(ns[from]);
+    return nt == 64    ? one(std::integral_constant<int, 64>{}, long_first, on, from, to)
+           : nt == 128 ? one(std::integral_constant<int, 128>{}, long_first, on, from, to)
+                       : one(std::integral_constant<int, 256>{}, long_first, on, from, to);
   };
   cudaError_t e = cudaSuccess;
-  if (overlap) {
-    for (int to = count, from; to > 0 && e == cudaSuccess; to = from) {
-      for (from = to - 1; from > 0 && threads_of(ns[from - 1]) == threads_of(ns[to - 1]);) --from;
-      e = run(from, to);
-    }
-  } else {
+  const bool classes = std::any_of(ns.begin(), ns.end(), [&](int n) { return threads_of(n) != threads_of(ns[0]); });
+  if (fork == nullptr || !classes) {
     for (int from = 0, to; from < count && e == cudaSuccess; from = to) {
       for (to = from + 1; to < count && threads_of(ns[to]) == threads_of(ns[from]);) ++to;
-      e = run(from, to);
+      e = run(std::false_type{}, st, from, to);
     }
+    return e;
+  }
+  if ((e = fork->create()) != cudaSuccess || (e = cudaEventRecord(fork->begin, st)) != cudaSuccess) return e;
+  int used = 0;  // forked streams
+  for (int to = count, from, c = 0; to > 0; to = from, ++c) {
+    for (from = to - 1; from > 0 && threads_of(ns[from - 1]) == threads_of(ns[to - 1]);) --from;
+    const int k = (c - 1) % LuFork::kStreams;
+    if (c > 0 && c <= LuFork::kStreams) {
+      if ((e = cudaStreamWaitEvent(fork->s[k], fork->begin, 0)) != cudaSuccess) return e;
+      used = c;
+    }
+    if ((e = run(std::true_type{}, c == 0 ? st : fork->s[k], from, to)) != cudaSuccess) return e;
+  }
+  for (int k = 0; k < used; ++k) {
+    if ((e = cudaEventRecord(fork->end[k], fork->s[k])) != cudaSuccess) return e;
+    if ((e = cudaStreamWaitEvent(st, fork->end[k], 0)) != cudaSuccess) return e;
   }
   return e;
 }
@@ -1538,7 +1527,7 @@ cudaError_t run_phases(cudaStream_t st, const BItem<C, typename Wide<C>::type> *
                        int max_s, int *d_info, const std::vector<int> &ns,
                        const std::vector<BPlan> &pls, const int *d_prefix128 = nullptr, int tiles128 = 0,
                        int *d_err = nullptr, int tc_first = 0, int tiles_simt = 0,
-                       const int *lu_threads = nullptr) {
+                       LuFork *fork = nullptr, const int *lu_threads = nullptr) {
   using W = typename Wide<C>::type;
   cudaError_t e;
   const dim3 ew((unsigned)count, (unsigned)((max_n * max_n + kEwChunk - 1) / kEwChunk));
@@ -1571,7 +1560,7 @@ cudaError_t run_phases(cudaStream_t st, const BItem<C, typename Wide<C>::type> *
   if ((e = gemm(kPhU, 1)) != cudaSuccess) return e;
   b_split_kernel<C, W><<<ew, 256, 0, st>>>(d_items);
   if ((e = launched()) != cudaSuccess) return e;
-  if ((e = launch_lu<BItem<C, W>, C, ExpmLu, true>(st, d_items, d_plans, d_info, 0, ns, lu_threads)) !=
+  if ((e = launch_lu<BItem<C, W>, C, ExpmLu, true>(st, d_items, d_plans, d_info, 0, ns, fork, lu_threads)) !=
       cudaSuccess)
     return e;
   if (max_s > 0) {
@@ -1611,6 +1600,22 @@ cudaError_t side_stream(calamanHandle_t blas, bool want, cudaStream_t &side) {
   }
   side = blas->side;
   return cudaSuccess;
+}
+
+// The forked streams of the LU's size classes: one set for the FP32 matrices, one
+// for the FP64 ones, which may run at the same time. Calls of up to kForkItems
+// matrices of both precisions, some four to sixteen CTAs per SM; null beyond, and
+// without a handle to hold the streams. Plain against forked, us a call, n = 3 .. 200
+// and norms 0.1 .. 100: float64 60 matrices 1351 -> 913, 500 2675 -> 2127, 1184 4448 ->
+// 3888, 2048 7079 -> 6385; float32 (a mixed batch) 500 2335 -> 1793, 2048 4785 -> 4647,
+// 3000 6757 -> 6804, 8192 18224 -> 18533: thousands fill every launch nearly to its end.
+// (As programmatic dependent launches in one stream, whose CTAs wait at their end for
+// the class before and hold their SM's slots meanwhile, 500 float64 took 2311, and the
+// 8192 matrices in 16 sub-batches on 16 streams 233.9k expm/s from and to the host,
+// against 266k plain and 274k so.)
+constexpr int kForkItems = 16 * 148;
+LuFork *lu_fork(calamanHandle_t blas, int fp64, int batch) {
+  return blas != nullptr && batch <= kForkItems ? &blas->lu_fork[fp64] : nullptr;
 }
 
 // Fork (before) or join (after) the side stream around a call's launches.
@@ -1775,7 +1780,7 @@ calamanStatus_t batched_api(calamanHandle_t blas, calamanStream_t stream, int ba
       b_conv_kernel<T, Hi><<<ew, 256, 0, sh>>>(d_cin);
       if ((e = launched()) != cudaSuccess) return e;
       if ((e = run_phases<Hi>(sh, d_hi, d_phi, d_xhi, nhi, hi_prefix.back(), hi_max_n, hi_max_s, d_info, hi_n,
-                              hi_plans, nullptr, 0, nullptr, 0, 0, tune.lu_threads)) != cudaSuccess)
+                              hi_plans, nullptr, 0, nullptr, 0, 0, lu_fork(blas, 1, batch), tune.lu_threads)) != cudaSuccess)
         return e;
       b_conv_kernel<Hi, T><<<ew, 256, 0, sh>>>(d_cout);
       if ((e = launched()) != cudaSuccess) return e;
@@ -1783,7 +1788,7 @@ calamanStatus_t batched_api(calamanHandle_t blas, calamanStream_t stream, int ba
     if (nlo > 0 &&
         (e = run_phases<T>(st, d_lo, d_plo, d_xlo, nlo, lo_prefix.back(), lo_max_n, lo_max_s, d_info, lo_n,
                            lo_plans, tc ? d_x128 : nullptr, tc_prefix.back(), d_err, tc_first,
-                           lo_prefix[tc_first], tune.lu_threads)) != cudaSuccess)
+                           lo_prefix[tc_first], lu_fork(blas, 0, batch), tune.lu_threads)) != cudaSuccess)
       return e;
     return side_join(blas, st, side);
   };
@@ -2124,7 +2129,7 @@ cudaError_t run_vjp_phases(cudaStream_t st, const BVItem<C, typename Wide<C>::ty
                            const BPlan *d_plans, const int *d_prefix, int count, int tiles, int max_n,
                            int max_s, int *d_info, const std::vector<int> &ns,
                            const std::vector<BPlan> &pls, const int *d_prefix128 = nullptr, int tiles128 = 0,
-                           int *d_err = nullptr, int tc_first = 0, int tiles_simt = 0) {
+                           int *d_err = nullptr, int tc_first = 0, int tiles_simt = 0, LuFork *fork = nullptr) {
   using W = typename Wide<C>::type;
   using Item = BVItem<C, W>;
   cudaError_t e;
@@ -2177,9 +2182,9 @@ cudaError_t run_vjp_phases(cudaStream_t st, const BVItem<C, typename Wide<C>::ty
   if ((e = gemm(kPhU, 2)) != cudaSuccess) return e;
   v_split_kernel<C, W><<<ew, 256, 0, st>>>(d_items);
   if ((e = launched()) != cudaSuccess) return e;
-  if ((e = launch_lu<Item, C, VjpLu, true>(st, d_items, d_plans, d_info, 0, ns)) != cudaSuccess) return e;
+  if ((e = launch_lu<Item, C, VjpLu, true>(st, d_items, d_plans, d_info, 0, ns, fork)) != cudaSuccess) return e;
   if ((e = gemm(kPhRhs, 1)) != cudaSuccess) return e;
-  if ((e = launch_lu<Item, C, VjpLu, false>(st, d_items, d_plans, d_info, 1, ns)) != cudaSuccess) return e;
+  if ((e = launch_lu<Item, C, VjpLu, false>(st, d_items, d_plans, d_info, 1, ns, fork)) != cudaSuccess) return e;
   if (max_s > 0) {
     v_widen_kernel<C, W><<<ew, 256, 0, st>>>(d_items, d_plans);
     if ((e = launched()) != cudaSuccess) return e;
@@ -2366,7 +2371,7 @@ calamanStatus_t vjp_batched_api(calamanHandle_t blas, calamanStream_t stream, in
     b_conv_kernel<T, Hi><<<dim3((unsigned)nin, chunks), 256, 0, sh>>>(d_conv);
     CLM_CUDA(launched());
     CLM_CUDA(run_vjp_phases<Hi>(sh, d_hi, d_phi, d_xhi, nhi, hi_prefix.back(), hi_max_n, hi_max_s, d_info,
-                                hi_n, hi_plans));
+                                hi_n, hi_plans, nullptr, 0, nullptr, 0, 0, lu_fork(blas, 1, batch)));
     b_conv_kernel<Hi, T><<<dim3((unsigned)nout, chunks), 256, 0, sh>>>(d_conv + nin);
     CLM_CUDA(launched());
   }
@@ -2390,7 +2395,7 @@ calamanStatus_t vjp_batched_api(calamanHandle_t blas, calamanStream_t stream, in
     }
     CLM_CUDA(run_vjp_phases<T>(st, d_lo, d_plo, d_xlo, nlo, lo_prefix.back(), lo_max_n, lo_max_s, d_info,
                                lo_n, lo_plans, tc ? d_x128 : nullptr, tc_prefix.back(), d_err, tc_first,
-                               lo_prefix[tc_first]));
+                               lo_prefix[tc_first], lu_fork(blas, 0, batch)));
   }
   CLM_CUDA(side_join(blas, st, side));
   return ok_status();

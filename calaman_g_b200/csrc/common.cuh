@@ -336,6 +336,30 @@ struct BatchedGraph {
   unsigned launches = 0;        // kernels in the graph (counted again at every replay)
 };
 
+// Streams for the size classes of a small batch's LU, forked from and joined to the
+// stream of the call, created on first use.
+struct LuFork {
+  static constexpr int kStreams = 2;
+  cudaStream_t s[kStreams] = {};
+  cudaEvent_t begin = nullptr, end[kStreams] = {};
+  cudaError_t create() {
+    cudaError_t e = cudaSuccess;
+    if (begin == nullptr) e = cudaEventCreateWithFlags(&begin, cudaEventDisableTiming);
+    for (int k = 0; k < kStreams && e == cudaSuccess; ++k) {
+      if (end[k] == nullptr) e = cudaEventCreateWithFlags(&end[k], cudaEventDisableTiming);
+      if (e == cudaSuccess && s[k] == nullptr) e = cudaStreamCreateWithFlags(&s[k], cudaStreamNonBlocking);
+    }
+    return e;
+  }
+  void destroy() {
+    for (int k = 0; k < kStreams; ++k) {
+      if (s[k]) cudaStreamDestroy(s[k]);
+      if (end[k]) cudaEventDestroy(end[k]);
+    }
+    if (begin) cudaEventDestroy(begin);
+  }
+};
+
 }  // namespace clm
 
 // The opaque handle behind calamanHandle_t.
@@ -359,5 +383,6 @@ struct calamanContext {
   // beside the FP32 ones) and the fork / join events, created on first use
   cudaStream_t side = nullptr;
   cudaEvent_t side_fork = nullptr, side_join = nullptr;
+  clm::LuFork lu_fork[2];      // of a batched call's FP32 and FP64 matrices
   clm::KernelTimer timer;
 };

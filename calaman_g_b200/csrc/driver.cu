@@ -476,6 +476,7 @@ calamanStatus_t calamanDestroy(calamanHandle_t handle) {
   if (handle->side) cudaStreamDestroy(handle->side);
   if (handle->side_fork) cudaEventDestroy(handle->side_fork);
   if (handle->side_join) cudaEventDestroy(handle->side_join);
+  for (auto &f : handle->lu_fork) f.destroy();
   delete handle;
   return ok_status();
 }

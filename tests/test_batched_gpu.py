@@ -183,3 +183,36 @@ def test_schedule_setting_and_the_tuner(run, oracle):
         assert st.ok and all(rel_frob(e.astype(np.float64), r) <= SINGLE_REL for e, r in zip(o32, ref))
     finally:
         run.lib.calamanSetBatchedTuning(run.h, (ctypes.c_int * 17)(*default[0]), default[1])
+
+
+@pytest.mark.parametrize("suf", ["s", "d"])
+@pytest.mark.parametrize("zigzag", [False, True])
+def test_forked_lu_classes_match_plain_launches(run, suf, zigzag):
+    """A small batch runs the size classes of its LU on forked streams, a call without a handle and one of
+    thousands of matrices run them one after the other: the same bits, and again when the call's graph is
+    replayed. zigzag: a schedule of five runs of CTA sizes, more than there are streams."""
+    import copy
+    import ctypes
+
+    lu, tc = (ctypes.c_int * 17)(), ctypes.c_int()
+    assert run.lib.calamanGetBatchedTuning(run.h, lu, ctypes.byref(tc)).ok
+    dt = np.float32 if suf == "s" else np.float64
+    mats = [m.astype(dt) for m in mixed_batch(600) + c4_batch(60, 601)]
+    ones = [np.full((1, 1), 0.01 * (i % 90), dtype=dt) for i in range(2400)]
+    try:
+        if zigzag:
+            sched = [64, 64, 256, 64] + [128] * 5 + [256] * 8
+            assert run.lib.calamanSetBatchedTuning(run.h, (ctypes.c_int * 17)(*sched), tc.value).ok
+        st, _, plain, _, info = run.batched(mats + ones, suf)
+        assert st.ok and (info == 0).all()
+        for _ in range(3):  # directly, captured, replayed
+            st, _, outs, _, info = run.batched(mats, suf)
+            assert st.ok and (info == 0).all()
+            assert all(np.array_equal(a, b) for a, b in zip(outs, plain))
+        if not zigzag:
+            bare = copy.copy(run)
+            bare.h = None
+            st, _, outs, _, _ = bare.batched(mats, suf)
+            assert st.ok and all(np.array_equal(a, b) for a, b in zip(outs, plain))
+    finally:
+        run.lib.calamanSetBatchedTuning(run.h, lu, tc.value)

@@ -81,3 +81,20 @@ def test_padding_and_argument_checks(run):
     assert all(np.all(d == -123.5) for d in grads)
     st, *_ = run_vjp_batched(run, pairs, "d", lwork=256)
     assert st.code == run.capi.ALLOC_FAILED
+
+
+@pytest.mark.parametrize("suf", ["s", "d"])
+def test_forked_lu_classes_match_plain_launches(run, suf):
+    """The two LU phases of a small batch on forked streams and, without a handle, one class after the other."""
+    import copy
+
+    pairs = pairs_of([(3, 0.5), (40, 3.0), (64, 20.0), (65, 1.0), (100, 6.0), (130, 0.8), (200, 15.0), (17, 2.0)], 920)
+    dt = np.float32 if suf == "s" else np.float64
+    pairs = [(a.astype(dt), g.astype(dt)) for a, g in pairs]
+    bare = copy.copy(run)
+    bare.h = None
+    st, _, plain, pe, _, info = run_vjp_batched(bare, pairs, suf)
+    assert st.ok and (info == 0).all()
+    st, _, grads, exps, _, info = run_vjp_batched(run, pairs, suf)
+    assert st.ok and (info == 0).all()
+    assert all(np.array_equal(a, b) for a, b in zip(grads + exps, plain + pe))
