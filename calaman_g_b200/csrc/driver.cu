@@ -171,9 +171,9 @@ calamanStatus_t expm_api(calamanHandle_t blas, calamanStream_t stream, int n, co
   if (plan_out) *plan_out = chosen;
 
   // Small matrices: everything after the norm in one kernel, faster than the
-  // general path's launches even as a graph (see small.cu). Not while GEMM
-  // launches are being timed, since it has none.
-  if (n <= expm_small_max_n<T>() && tl_timer == nullptr) {
+  // general path's launches even as a graph (see small.cu). It has no GEMM launch
+  // to time, and is the same with kernel timing on.
+  if (n <= expm_small_max_n<T>()) {
     CLM_CUDA(expm_small<T>(st, n, A, lda, E, lde, chosen.m, chosen.s, d_info));
     return ok_status();
   }

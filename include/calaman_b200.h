@@ -629,8 +629,9 @@ calamanStatus_t calaman_getrf_wait_check_z(calamanStream_t stream, int n, void *
 unsigned long long calamanGetLaunchCount(void);
 
 /* Per-handle CUDA-event timing of the dense products (every GEMM launch the
- * handle's calls issue, including those inside the LU and the solves).
- * Enabling clears the record; reading synchronises on the last event. */
+ * handle's calls issue, including those inside the LU and the solves). A call
+ * of calaman_expm_* for n <= 64 (complex 48) is one kernel behind the norm and
+ * has no such launch. Timing changes no result. Enabling clears the record; reading synchronises on the last event. */
 typedef struct {
   long long gemm_launches;
   double gemm_ms;        /* summed device time of those launches */

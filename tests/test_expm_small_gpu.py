@@ -77,3 +77,18 @@ def test_small_expm_in_place(run, oracle, suf, norm):
     assert np.array_equal(full.reshape(n, ld)[:, n:], before)  # the padding rows are untouched
     ref, _, _ = oracle.expm(a, single=suf in "sc")
     assert rel_frob(from_buffer(full, n, ld), ref) <= BAR[suf]
+
+
+@pytest.mark.parametrize("suf", ["s", "d", "c", "z"])
+def test_kernel_timing_runs_the_same_kernel(run, suf):
+    """With kernel timing on a small matrix takes the same path: the same bits, and no GEMM launch to time."""
+    a = scaled_random(37, 2.0, 6, suf in "cz").astype(NP_DTYPE[suf])
+    st, _, plain, _, _ = run.expm(a, suf)
+    assert st.ok and run.lib.calamanSetKernelTiming(run.h, 1).ok
+    try:
+        st, _, timed, _, info = run.expm(a, suf)
+        kt = run.capi.KernelTiming()
+        assert st.ok and list(info) == [0, 0] and run.lib.calamanGetKernelTiming(run.h, ctypes.byref(kt)).ok
+    finally:
+        run.lib.calamanSetKernelTiming(run.h, 0)
+    assert np.array_equal(timed, plain) and kt.gemm_launches == 0
