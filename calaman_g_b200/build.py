@@ -36,7 +36,7 @@ def sources() -> list[str]:
 
 
 def _deps(src: str) -> list[str]:
-    hdrs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
+    hdrs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h", ".hpp"))]
     hdrs.append(os.path.join(HERE, "..", "include", "calaman_b200.h"))
     return [src] + hdrs
 

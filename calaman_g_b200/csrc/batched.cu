@@ -860,13 +860,10 @@ inline int tiles128_of(int n) {
 template <typename Item, typename Ops>
 cudaError_t launch_group_tc(cudaStream_t st, dim3 grid, const Item *items, const BPlan *plans,
                             const int *prefix128, int count, int phase, int *err) {
-  static bool configured = false;
+  static OncePerDevice once;
   auto kern = g_tc_kernel<Item, Ops>;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  const cudaError_t e = opt_in_smem(once, kern, kTcSmem);
+  if (e != cudaSuccess) return e;
   kern<<<grid, kTcThreads, kTcSmem, st>>>(items, plans, prefix128, count, phase, err);
   return launched();
 }
@@ -877,13 +874,10 @@ template <typename Item, typename U, typename Ops, bool kSquare>
 cudaError_t launch_group(cudaStream_t st, dim3 grid, const Item *items, const BPlan *plans,
                          const int *prefix, int count, int phase, int k) {
   if constexpr (std::is_same<U, double>::value) {
-    static bool configured = false;
+    static OncePerDevice once;
     auto kern = g_dgemm_kernel<Item, Ops, kSquare>;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDSmem);
-      if (e != cudaSuccess) return e;
-      configured = true;
-    }
+    const cudaError_t e = opt_in_smem(once, kern, kDSmem);
+    if (e != cudaSuccess) return e;
     kern<<<grid, 128, kDSmem, st>>>(items, plans, prefix, count, phase, k);
   } else {
     g_gemm_kernel<Item, U, Ops, kSquare><<<grid, 256, 0, st>>>(items, plans, prefix, count, phase, k);
@@ -1334,15 +1328,10 @@ cudaError_t launch_lu(cudaStream_t st, const Item *items, const BPlan *plans, in
     constexpr int NT = decltype(nt_tag)::value;
     auto kern = g_lu_kernel<Item, T, Lu, kFactor, NT, decltype(long_first)::value>;
     constexpr std::size_t smem = lu_smem_bytes<T, NT>();
-    static bool configured = false;  // once, before any graph capture of a call
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      // the largest shared-memory carveout, so the CTAs the registers allow fit
-      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-      if (e != cudaSuccess) return e;
-      configured = true;
-    }
+    static OncePerDevice once;
+    // the largest shared-memory carveout, so the CTAs the registers allow fit
+    const cudaError_t e = opt_in_smem(once, kern, smem, 100);
+    if (e != cudaSuccess) return e;
     kern<<<to - from, NT, smem, on>>>(items + from, plans + from, info, mode);
     return launched();
   };

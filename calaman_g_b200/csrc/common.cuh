@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/calaman_b200.h"
+#include "once_per_device.hpp"
 
 namespace clm {
 
@@ -359,6 +360,21 @@ struct LuFork {
     if (begin) cudaEventDestroy(begin);
   }
 };
+
+// A kernel's dynamic shared memory beyond the default, once on the current device;
+// carveout: the preferred share of shared memory in percent (-1: the driver's).
+// One `once` per kernel.
+template <typename K>
+cudaError_t opt_in_smem(OncePerDevice &once, K kern, std::size_t bytes, int carveout = -1) {
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  return once.run(device, [&] {
+    const cudaError_t a = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (a != cudaSuccess || carveout < 0) return a;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
+  });
+}
 
 }  // namespace clm
 

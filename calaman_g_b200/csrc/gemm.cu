@@ -584,12 +584,9 @@ cudaError_t run_dgemm(cudaStream_t s, int M, int N, int K, double alpha, const d
   constexpr int NT = (BM / WM) * (BN / WN) * 32;
   constexpr int smem = STAGES * (16 * (BM + 4) + BN * 20) * (int)sizeof(double);
   auto kern = dgemm_nn_kernel<BM, BN, WM, WN, STAGES, V16>;
-  static bool configured = false;  // attribute is per-function, process-wide
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static OncePerDevice once;
+  const cudaError_t e = opt_in_smem(once, kern, smem);
+  if (e != cudaSuccess) return e;
   dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, splits);
   kern<<<grid, NT, smem, s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, splits > 1 ? kslice : K,
                               cstride);
@@ -603,12 +600,9 @@ cudaError_t run_zgemm(cudaStream_t s, int M, int N, int K, double alpha, const d
   constexpr int NT = (BM / WM) * (BN / WN) * 32;
   constexpr int smem = STAGES * (16 * (BM + 2) + BN * 20) * (int)sizeof(double2);
   auto kern = zgemm_nn_kernel<BM, BN, WM, WN, STAGES, kGauss>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static OncePerDevice once;
+  const cudaError_t e = opt_in_smem(once, kern, smem);
+  if (e != cudaSuccess) return e;
   dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, splits);
   kern<<<grid, NT, smem, s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, splits > 1 ? kslice : K,
                               cstride);

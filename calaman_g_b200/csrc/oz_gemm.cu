@@ -581,13 +581,8 @@ cudaError_t oz_gemm(cudaStream_t s, int M, int N, int K, double alpha, const T *
   p.spin = spin > 0 ? spin : kSpinLimit;
   p.skip_loads = skip_loads;
 
-  static bool configured = false;
-  if (!configured) {
-    if ((e = cudaFuncSetAttribute(oz_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOzSmem)) !=
-        cudaSuccess)
-      return e;
-    configured = true;
-  }
+  static OncePerDevice once;
+  if ((e = opt_in_smem(once, oz_gemm_kernel, kOzSmem)) != cudaSuccess) return e;
   oz_gemm_kernel<<<dim3(L.Mrp / OTM, L.Np / OTN), kOzThreads, kOzSmem, s>>>(ma, mb, p);
   if ((e = launched()) != cudaSuccess || !diag) return e;
   oz_diag_terms_kernel<T><<<dim3((M + 255) / 256, N), 256, 0, s>>>(M, alpha, A, lda, B, ldb, C, ldc);

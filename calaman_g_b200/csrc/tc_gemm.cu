@@ -553,12 +553,9 @@ cudaError_t tc_gemm_run(cudaStream_t s, int Mc, int N, int Kc, double alpha, con
     r.skip = skip;
     constexpr int smem = 6 * kPart + 1024;
     auto kern = tc_rank_kernel<cplx>;
-    static bool configured = false;
-    if (!configured) {
-      const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) return e;
-      configured = true;
-    }
+    static OncePerDevice once;
+    const cudaError_t e = opt_in_smem(once, kern, smem);
+    if (e != cudaSuccess) return e;
     kern<<<dim3((M + TM - 1) / TM, (N + RN - 1) / RN), kRankThreads, smem, s>>>(r);
     return launched();
   }
@@ -603,13 +600,8 @@ cudaError_t tc_gemm_run(cudaStream_t s, int Mc, int N, int Kc, double alpha, con
   p.err = err;
 
   constexpr int smem = kStages * (kA + kB) + 1024 + 256;
-  static bool configured = false;
-  if (!configured) {
-    if ((e = cudaFuncSetAttribute(tc_split_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) !=
-        cudaSuccess)
-      return e;
-    configured = true;
-  }
+  static OncePerDevice once;
+  if ((e = opt_in_smem(once, tc_split_gemm_kernel, smem)) != cudaSuccess) return e;
   tc_split_gemm_kernel<<<dim3(L.Mpad / TM, L.Npad / TN), kThreads, smem, s>>>(ma, mb, p);
   return launched();
 }

@@ -19,3 +19,13 @@ def test_cpp_header_compiles_links_and_runs(tmp_path):
     out = subprocess.run([str(exe)], capture_output=True, text=True)
     assert out.returncode == 0, out.stdout + out.stderr
     assert "header_check ok" in out.stdout
+
+
+def test_kernel_attributes_are_due_once_per_device(tmp_path):
+    """The rule behind every kernel's shared-memory opt-in, on the host: a second device is configured too."""
+    exe = tmp_path / "once_per_device_check"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Wextra", "-Werror",
+                    os.path.join(ROOT, "tests", "cpp", "once_per_device_check.cpp"), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert out.returncode == 0, out.stdout + out.stderr
+    assert "once_per_device_check ok" in out.stdout
