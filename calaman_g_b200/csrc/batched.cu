@@ -1964,10 +1964,13 @@ __global__ void __launch_bounds__(256) v_prep_kernel(const BVItem<T, Wd> *__rest
   }
 }
 
-// the Pade combinations of the powers (P) and of their derivatives (M)
+// The Pade combinations of the powers (P) and of their derivatives (M). Four CTAs
+// per SM (64 registers): at the 88 that the 16-byte pieces would take in float64,
+// two CTAs had too few loads in flight (300 matrices of n = 99 61 -> 86 us, and 62 so;
+// n = 100 64 -> 76, and 57 so).
 template <typename T, typename Wd>
-__global__ void __launch_bounds__(256) v_even_odd_kernel(const BVItem<T, Wd> *__restrict__ items,
-                                                         const BPlan *__restrict__ plans) {
+__global__ void __launch_bounds__(256, 4) v_even_odd_kernel(const BVItem<T, Wd> *__restrict__ items,
+                                                            const BPlan *__restrict__ plans) {
   using R = typename elem<T>::real;
   const BVItem<T, Wd> it = items[blockIdx.x];
   const BPlan pl = plans[blockIdx.x];
@@ -2034,22 +2037,25 @@ __global__ void __launch_bounds__(256) v_even_odd_kernel(const BVItem<T, Wd> *__
 template <typename T, typename Wd>
 __global__ void __launch_bounds__(256) v_split_kernel(const BVItem<T, Wd> *__restrict__ items) {
   const BVItem<T, Wd> it = items[blockIdx.x];
-  auto split = [](T *u, T *v, int n) {  // (u, v) <- (v + u, v - u)
-    ew_for<T>(u, n * n, [&](auto piece, int e) {
-      constexpr int W = decltype(piece)::value;
-      const Pack<W, T> a = ew_load<W>(u + e), c = ew_load<W>(v + e);
-      Pack<W, T> p, q;
+  // one loop over both pairs: four loads in flight per step (a loop per pair: 300
+  // float64 pairs of n = 99 54 us against 38, 131 of n = 51 16 against 11)
+  ew_for<T>(it.V, it.n * it.n, [&](auto piece, int e) {
+    constexpr int W = decltype(piece)::value;
+    const Pack<W, T> u = ew_load<W>(it.T1 + e), v = ew_load<W>(it.V + e);
+    const Pack<W, T> du = ew_load<W>(it.T2 + e), dv = ew_load<W>(it.LV + e);
+    Pack<W, T> p, q, dp, dq;
 #pragma unroll
-      for (int i = 0; i < W; ++i) {
-        p.e[i] = add(c.e[i], a.e[i]);
-        q.e[i] = sub(c.e[i], a.e[i]);
-      }
-      ew_store<W>(u + e, p);
-      ew_store<W>(v + e, q);
-    });
-  };
-  split(it.T1, it.V, it.n);
-  split(it.T2, it.LV, it.n);
+    for (int i = 0; i < W; ++i) {
+      p.e[i] = add(v.e[i], u.e[i]);
+      q.e[i] = sub(v.e[i], u.e[i]);
+      dp.e[i] = add(dv.e[i], du.e[i]);
+      dq.e[i] = sub(dv.e[i], du.e[i]);
+    }
+    ew_store<W>(it.T1 + e, p);
+    ew_store<W>(it.V + e, q);
+    ew_store<W>(it.T2 + e, dp);
+    ew_store<W>(it.LV + e, dq);
+  });
 }
 
 // s > 0: (wr, wl) = wide (R, dR)
