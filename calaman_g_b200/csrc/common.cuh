@@ -366,9 +366,15 @@ struct LuFork {
 // One `once` per kernel.
 template <typename K>
 cudaError_t opt_in_smem(OncePerDevice &once, K kern, std::size_t bytes, int carveout = -1) {
+  static const int devices = [] {
+    int n = 0;
+    return cudaGetDeviceCount(&n) == cudaSuccess ? n : 0;
+  }();
   int device = 0;
-  const cudaError_t e = cudaGetDevice(&device);
-  if (e != cudaSuccess) return e;
+  if (devices != 1) {  // a query per launch (0.2 us) only where there is a choice
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+  }
   return once.run(device, [&] {
     const cudaError_t a = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (a != cudaSuccess || carveout < 0) return a;
