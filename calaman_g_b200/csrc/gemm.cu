@@ -6,7 +6,9 @@
 //   double2  : complex128 as four real DMMA products per tile
 //              (Re += Ar Br - Ai Bi, Im += Ar Bi + Ai Br), operands read once
 //              as interleaved 16-byte pairs.
-//   float / float2 : register-tiled FP32 SIMT kernel (the plain single tier).
+//   float / float2 : register-tiled FP32 SIMT kernels (the plain single tier): 8 x 8
+//              outputs a thread for float, 4 x 4 for complex64 and shallow float
+//              products.
 //
 // Operands are staged global -> shared by cp.async in a multi-stage ring; all
 // edges (M, N, K not multiples of the tile) are zero-filled by the copy's
@@ -692,12 +694,22 @@ cudaError_t gemm_nn<double2>(cudaStream_t s, int M, int N, int K, double alpha, 
   });
 }
 
-// Thin products (fewer than 64 rows or columns: the LU's look-ahead update of
-// the next panel's 32 columns, the last blocks of the triangular solves) fill
-// few tensor-core tiles; they run on the SIMT kernel, one launch instead of two
-// split kernels and a tcgen05 GEMM (float32 4096 expm 34.3 -> 36.4 expm/s, the
-// same error against the FP64 oracle).
+// Thin products (fewer than 64 rows or columns: the LU's update of the next
+// panel's 32 columns in complex64, ragged last blocks of the solves) fill few
+// tensor-core tiles; they run on the SIMT kernels. Complex64 expm, SIMT against the
+// split-BF16 kernel of shallow products: n = 60 153 us against 181, 777 1858 against
+// 1891, 1500 3823 against 3869, level in between, the same error against 64 bits.
 inline bool thin_product(int M, int N) { return M < 64 || N < 64; }
+
+// FP32 SIMT products whose few depth steps do not pay for the sums of sgemm_nn_kernel's
+// four k groups and its larger C tile per thread take the 4 x 4 form. us a launch, 4 x 4
+// against 8 x 8: depth 16 at 16 x 16 2.3 / 5.0, at 200 x 200 4.3 / 5.5, at 1000 x 1000 6.9 /
+// 7.5; depth 32 at 200 x 200 5.2 / 5.5, at 1000 x 1000 8.6 / 7.6; depth 48 at 50 x 50 5.1 /
+// 6.2; depth 64 at 32 x 32 5.6 / 6.1, at 64 x 64 7.5 / 6.3, at 200 x 200 7.2 / 6.6.
+inline bool shallow_product(int M, int N, int K) {
+  const long long tiles = (long long)((M + 63) / 64) * ((N + 63) / 64);
+  return K <= 16 || (K < 64 && tiles <= 148) || (K <= 64 && M <= 32 && N <= 32);
+}
 
 template <>
 cudaError_t gemm_nn<float>(cudaStream_t s, int M, int N, int K, double alpha, const float *A,
@@ -712,6 +724,10 @@ cudaError_t gemm_nn<float>(cudaStream_t s, int M, int N, int K, double alpha, co
   }
   return timed_launch(s, real_flops(M, N, K), [&] {
     dim3 grid((M + 63) / 64, (N + 63) / 64);
+    if (shallow_product(M, N, K)) {
+      simt_gemm_nn_kernel<float><<<grid, 256, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+      return cudaGetLastError();
+    }
     const bool v16 = aligned16(A) && aligned16(B) && (lda % 4 == 0) && (ldb % 4 == 0);
     auto kern = v16 ? sgemm_nn_kernel<true> : sgemm_nn_kernel<false>;
     kern<<<grid, 256, 0, s>>>(M, N, K, (float)alpha, A, lda, B, ldb, (float)beta, C, ldc);
