@@ -10,9 +10,17 @@ from helpers import NP_DTYPE, Runner, _dev, colmajor_buffer, from_buffer, rel_fr
 
 pytestmark = pytest.mark.gpu
 
-# FP64 tiers: the library's bar. Single tiers: eps (6e-8) x the entries' growth in
-# the scaled evaluation (a few tens) x 2^s for the squarings of the quotient's error.
-BAR = {"d": 1e-12, "z": 1e-12, "s": 2e-5, "c": 2e-5}
+# FP64 tiers: the library's bar. Single tiers: the one kernel evaluates in FP64 and rounds each
+# entry once, so at most 2^-24 (6e-8) of the result's norm, and the oracle's FP64 beside it; FP32
+# arithmetic anywhere in it shows (1.8e-7 at norm 1). Sizes beyond the kernel take the general path,
+# with eps x the entries' growth in the scaled evaluation (a few tens) x 2^s for the squarings.
+BAR = {"d": 1e-12, "z": 1e-12, "s": 6.1e-8, "c": 6.1e-8}
+GENERAL = {"d": 1e-12, "z": 1e-12, "s": 2e-5, "c": 2e-5}
+NORMS = [0.01, 0.2, 0.9, 2.0, 3.5, 5.3, 40.0]  # m = 3 .. 13, s = 0 and s > 0
+
+
+def bar(suf, n):
+    return BAR[suf] if n <= (48 if suf in "cz" else 64) else GENERAL[suf]
 
 
 @pytest.fixture(scope="module")
@@ -23,8 +31,9 @@ def run(cuda):
 
 
 @pytest.mark.parametrize("suf", ["s", "d", "c", "z"])
-@pytest.mark.parametrize("n", [1, 2, 3, 15, 16, 17, 32, 33, 47, 48, 49, 63, 64, 65])
-@pytest.mark.parametrize("norm", [0.01, 0.2, 0.9, 2.0, 3.5, 5.3, 40.0])  # m = 3 .. 13, s = 0 and s > 0
+@pytest.mark.parametrize("n,norm", [(n, t) for n in (17, 48, 64) for t in NORMS]
+                         + [(n, NORMS[(i + k) % 7]) for i, n in enumerate((1, 2, 3, 15, 16, 32, 33, 47, 49, 63, 65))
+                            for k in (0, 2, 5)])
 def test_small_expm_matches_oracle(run, oracle, suf, n, norm):
     a = scaled_random(n, norm, 77 * n + int(10 * norm), suf in "cz")
     if norm > 6:
@@ -38,7 +47,7 @@ def test_small_expm_matches_oracle(run, oracle, suf, n, norm):
     ref, oplan, _ = oracle.expm(a, single=suf in "sc")
     assert st.ok and list(info) == [0, 0]
     assert (plan.m, plan.s) == (oplan.m, oplan.s)
-    assert rel_frob(e, ref) <= BAR[suf]
+    assert rel_frob(e, ref) <= bar(suf, n)
 
 
 @pytest.mark.parametrize("suf", ["d", "z"])
@@ -76,7 +85,7 @@ def test_small_expm_in_place(run, oracle, suf, norm):
     full = dA.cpu().numpy()
     assert np.array_equal(full.reshape(n, ld)[:, n:], before)  # the padding rows are untouched
     ref, _, _ = oracle.expm(a, single=suf in "sc")
-    assert rel_frob(from_buffer(full, n, ld), ref) <= BAR[suf]
+    assert rel_frob(from_buffer(full, n, ld), ref) <= bar(suf, n)
 
 
 @pytest.mark.parametrize("suf", ["s", "d", "c", "z"])

@@ -64,7 +64,7 @@ def test_getrf_matches_oracle_exactly_in_pivots(lib, oracle, suf, n):
 
 
 @pytest.mark.parametrize("suf", ["s", "c"])
-@pytest.mark.parametrize("n", [5, 64, 200, 700, 3001])  # 3001: the tallest one-CTA panel class
+@pytest.mark.parametrize("n", [5, 64, 200, 700, 3001])
 def test_getrf_single_backward_error(lib, suf, n):
     a = gaussian(n, suf, 600 + n)
     _, _, lu, ipiv, info = run_getrf(lib, a, suf)
@@ -138,6 +138,43 @@ def test_pade_large_norm_pivoting(oracle, suf, m, target, cuda):
     run.close()
     assert st.ok and list(info) == [0, 0]
     assert rel_frob(r, ref) <= (1e-11 if suf in "dz" else 1e-3)
+
+
+@pytest.mark.parametrize("suf", ["s", "d", "c", "z"])
+@pytest.mark.parametrize("n", [600, 1100])
+def test_solve_beside_the_factorisation_pivots(cuda, suf, n):
+    """pade() solves beside its LU. A has imaginary eigenvalues close to pi and a dense orthogonal (unitary)
+    basis, so q_13 is close to a multiple of exp(-A/2), a dense orthogonal matrix with a small diagonal:
+    perfectly conditioned, and most of its columns pivot, in panels of eight CTAs and of one, with the
+    look-ahead and the right-hand side's swaps and updates. r_13 is exp(A) to rounding at this norm."""
+    import torch
+
+    from helpers import Runner, rel_frob
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    wide = torch.complex128 if suf in "cz" else torch.float64
+    q, _ = torch.linalg.qr(torch.randn(n, n, generator=g, dtype=wide, device="cuda"))
+    w = 3.05 + 0.18 * torch.rand(n // 2, generator=g, dtype=torch.float64, device="cuda")
+    if suf in "cz":
+        k = torch.diag(torch.cat([1j * w, -1j * w]))
+    else:
+        k = torch.zeros(n, n, dtype=wide, device="cuda")
+        i = torch.arange(0, n, 2, device="cuda")
+        k[i, i + 1], k[i + 1, i] = w, -w
+    a = (q @ k @ q.mH).to({"s": torch.float32, "c": torch.complex64}.get(suf, wide))
+    den, num = torch.linalg.matrix_exp(a.to(wide) / -2), torch.linalg.matrix_exp(a.to(wide) / 2)
+    pivots = torch.linalg.lu_factor(den)[1].cpu().numpy()
+    assert (pivots != np.arange(1, n + 1)).sum() > n // 2
+    run = Runner()
+    st, r, info = run.pade(a.cpu().numpy(), 13, suf)
+    run.close()
+    assert st.ok and list(info) == [0, 0]
+    ref = torch.linalg.matrix_exp(a.to(wide)).cpu().numpy()
+    # a dense orthogonal matrix has element growth (77 at n = 600, 156 at 1100) that any LU with partial
+    # pivoting shows: four times the error of torch's own in this precision (1.9e-5 in float32 at 1100), and
+    # a few tens of roundings for the products behind q and p
+    other = rel_frob(torch.linalg.solve(den.to(a.dtype), num.to(a.dtype)).cpu().numpy(), ref)
+    assert rel_frob(r, ref) <= 4 * other + 64 * eps(suf)
 
 
 def hadamard(n):
