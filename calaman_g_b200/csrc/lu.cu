@@ -653,11 +653,11 @@ inline cudaLaunchAttribute cluster_attr(int ncta) {
   return a;
 }
 
-// One row per thread: one CTA up to 512 rows, where the exchange between CTAs
-// costs more than the warps that share an SM (a float64 column of 512 rows:
-// 1.09 us in one CTA, 1.22 to 1.28 in 2 to 8); above, always eight CTAs, since
-// fewer rows per SM shorten the update (float64, 2048 rows: 1.54 us a column on
-// four CTAs, 1.37 on eight).
+// One row per thread: one CTA up to MAXT rows (512; 256 for complex128 factorisations
+// of n <= 2048), where the exchange between CTAs costs more than the warps that share
+// an SM (a float64 column of 512 rows: 1.09 us in one CTA, 1.22 to 1.28 in 2 to 8);
+// above, always eight CTAs, since fewer rows per SM shorten the update (float64,
+// 2048 rows: 1.54 us a column on four CTAs, 1.37 on eight).
 template <typename T, int KB, int MAXT>
 cudaError_t launch_rows_panel(cudaStream_t s, int n, T *A, int lda, int k, int kb, const LuScratch &sc,
                               const RowMap &map, int *info, const PanelWait &wait) {
