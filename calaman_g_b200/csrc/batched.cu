@@ -1352,18 +1352,19 @@ cudaError_t launch_lu(cudaStream_t st, const Item *items, const BPlan *plans, in
   }
   if ((e = fork->create()) != cudaSuccess || (e = cudaEventRecord(fork->begin, st)) != cudaSuccess) return e;
   int used = 0;  // forked streams
-  for (int to = count, from, c = 0; to > 0; to = from, ++c) {
+  for (int to = count, from, c = 0; to > 0 && e == cudaSuccess; to = from, ++c) {
     for (from = to - 1; from > 0 && threads_of(ns[from - 1]) == threads_of(ns[to - 1]);) --from;
     const int k = (c - 1) % LuFork::kStreams;
     if (c > 0 && c <= LuFork::kStreams) {
-      if ((e = cudaStreamWaitEvent(fork->s[k], fork->begin, 0)) != cudaSuccess) return e;
+      if ((e = cudaStreamWaitEvent(fork->s[k], fork->begin, 0)) != cudaSuccess) break;
       used = c;
     }
-    if ((e = run(std::true_type{}, c == 0 ? st : fork->s[k], from, to)) != cudaSuccess) return e;
+    e = run(std::true_type{}, c == 0 ? st : fork->s[k], from, to);
   }
-  for (int k = 0; k < used; ++k) {
-    if ((e = cudaEventRecord(fork->end[k], fork->s[k])) != cudaSuccess) return e;
-    if ((e = cudaStreamWaitEvent(st, fork->end[k], 0)) != cudaSuccess) return e;
+  for (int k = 0; k < used; ++k) {  // after an error too: the call's stream stays behind what was launched
+    cudaError_t j = cudaEventRecord(fork->end[k], fork->s[k]);
+    if (j == cudaSuccess) j = cudaStreamWaitEvent(st, fork->end[k], 0);
+    if (e == cudaSuccess) e = j;
   }
   return e;
 }
