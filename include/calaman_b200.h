@@ -191,7 +191,8 @@ calamanStatus_t calaman_expm_vjp_z(calamanBlasHandle_t blas, calamanSolverHandle
  * with s_i = 0 in FP32 and those with s_i > 0 wholly in FP64. When a batch
  * holds both, the FP64 ones run on a second stream that the blas handle
  * creates on first use (non-blocking, forked from and joined back to `stream`
- * within the call, released by calamanDestroy). */
+ * within the call, released by calamanDestroy). So do the size classes of the LU
+ * in calls of up to 2368 matrices. */
 calamanStatus_t calaman_expm_batched_bufferSize_s(calamanSolverHandle_t h, int batch,
                                                   const int *h_n, size_t *bytes);
 calamanStatus_t calaman_expm_batched_bufferSize_d(calamanSolverHandle_t h, int batch,
